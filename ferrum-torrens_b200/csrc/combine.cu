@@ -62,6 +62,11 @@ __global__ void cast_to_bf16_kernel(const void* __restrict__ src, int src_dtype,
 //   var = mean(f32(s)^2)                         f32
 //   y = bf16((f32(s) * (1 / sqrt(var + eps))) * f32(w))      w is the baked 1 + weight vector
 // One warp per row; a lane keeps its elements in registers between the two passes.
+__device__ __forceinline__ uint4 ld_in_order(const void* p) {      // issued where it stands
+    uint4 v;
+    asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+    return v;
+}
 template <int kPerLane>
 __global__ void __launch_bounds__(128)
 add_rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ r,
@@ -69,16 +74,25 @@ add_rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
                    __nv_bfloat16* __restrict__ sum_out, __nv_bfloat16* __restrict__ out) {
     const int row = blockIdx.x * 4 + threadIdx.x / 32, lane = threadIdx.x % 32;
     if (row >= tokens) return;
-    // chunk c of the lane: eight consecutive elements at (c * 32 + lane) * 8
+    // chunk c of the lane: eight consecutive elements at (c * 32 + lane) * 8.  All loads are issued before the first
+    // use (a few rows are one cold round trip to HBM; the weight row asked for after the reduction was a second one).
+    uint4 xv[kPerLane], rv[kPerLane], wv[kPerLane];
+#pragma unroll
+    for (int c = 0; c < kPerLane; c++) {
+        const int k = (c * 32 + lane) * 8;
+        if (k < H) {
+            xv[c] = ld_in_order(x + (size_t)row * H + k);
+            rv[c] = ld_in_order(r + (size_t)row * H + k);
+            if (kPerLane <= 8) wv[c] = ld_in_order(w + k);     // (sixteen chunks leave no registers for it)
+        }
+    }
     float sf[kPerLane][8];
     float ss = 0.f;
 #pragma unroll
     for (int c = 0; c < kPerLane; c++) {
         const int k = (c * 32 + lane) * 8;
         if (k < H) {
-            const uint4 xv = *reinterpret_cast<const uint4*>(x + (size_t)row * H + k);
-            const uint4 rv = *reinterpret_cast<const uint4*>(r + (size_t)row * H + k);
-            const uint32_t xw[4] = {xv.x, xv.y, xv.z, xv.w}, rw[4] = {rv.x, rv.y, rv.z, rv.w};
+            const uint32_t xw[4] = {xv[c].x, xv[c].y, xv[c].z, xv[c].w}, rw[4] = {rv[c].x, rv[c].y, rv[c].z, rv[c].w};
             uint32_t sw[4];
 #pragma unroll
             for (int q = 0; q < 4; q++) {
@@ -101,8 +115,8 @@ add_rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
     for (int c = 0; c < kPerLane; c++) {
         const int k = (c * 32 + lane) * 8;
         if (k < H) {
-            const uint4 wv = *reinterpret_cast<const uint4*>(w + k);
-            const uint32_t ww[4] = {wv.x, wv.y, wv.z, wv.w};
+            if (kPerLane > 8) wv[c] = ld_in_order(w + k);
+            const uint32_t ww[4] = {wv[c].x, wv[c].y, wv[c].z, wv[c].w};
             uint32_t yw[4];
 #pragma unroll
             for (int q = 0; q < 4; q++) {
