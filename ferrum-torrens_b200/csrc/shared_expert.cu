@@ -110,7 +110,6 @@ shared_phase2_kernel(const float* __restrict__ ic2s, int tokens, int H, int SI,
 // dimension (eight per tile).  A lane reads 16 contiguous bytes of a weight row (eight k) and the
 // same eight k of its token row; the k slots of two MMAs are fed from those eight k in order, for
 // both operands alike, so any assignment is consistent.  Each weight byte is read once.
-constexpr int kMaxTokTiles = 8;  // up to 64 tokens per pass
 
 __device__ __forceinline__ void mma_bf16_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
                                                uint32_t b0, uint32_t b1) {
@@ -120,55 +119,100 @@ __device__ __forceinline__ void mma_bf16_16816(float (&c)[4], uint32_t a0, uint3
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// partial products of one warp: rows (row_lo + g8, row_hi + g8) x tokens [tok0, tok0 + 8*NT) over
-// k in [k_begin, k_end), 32 k per step
+// Partial products of one warp: rows (row_lo + g8, row_hi + g8) x tokens [tok0, tok0 + 8*NT) over the k of [k_begin,
+// k_end), 32 k per step, SB steps at a time: the weight rows of a block of steps are all asked for before the first
+// is used (for a decode batch these kernels are one cold read of a few KB per warp, so they cost its latency: asking
+// for two steps at a time took 9.5 us per kernel), the tokens' rows UB steps at a time (they come from L2).
+template <int NT, int SB, int UB>
+__device__ __forceinline__ void load_rows(uint4 (&lo)[SB], uint4 (&hi)[SB], const __nv_bfloat16* __restrict__ w_lo,
+                                          const __nv_bfloat16* __restrict__ w_hi, int k, int k_end) {
+#pragma unroll
+    for (int i = 0; i < SB; i++)
+        if (k + i * 32 < k_end) {
+            lo[i] = *reinterpret_cast<const uint4*>(w_lo + k + i * 32);
+            hi[i] = *reinterpret_cast<const uint4*>(w_hi + k + i * 32);
+        }
+}
+template <int NT, int SB, int UB>
+__device__ __forceinline__ void mma_rows(const uint4 (&lo)[SB], const uint4 (&hi)[SB], const __nv_bfloat16* __restrict__ x,
+                                         int ldx, int tok0, int tokens, int k, int k_end, int g8, float (&acc)[NT][4]) {
+    const uint4 zero = make_uint4(0, 0, 0, 0);
+#pragma unroll
+    for (int i0 = 0; i0 < SB; i0 += UB) {
+        uint4 b[UB][NT];
+#pragma unroll
+        for (int i = 0; i < UB; i++)
+#pragma unroll
+            for (int n = 0; n < NT; n++) {
+                const int t = tok0 + n * 8 + g8, kk = k + (i0 + i) * 32;
+                b[i][n] = (t < tokens && kk < k_end) ? *reinterpret_cast<const uint4*>(x + (size_t)t * ldx + kk) : zero;
+            }
+#pragma unroll
+        for (int i = 0; i < UB; i++)
+            if (k + (i0 + i) * 32 < k_end) {
+                const uint4 &l = lo[i0 + i], &h = hi[i0 + i];
+#pragma unroll
+                for (int n = 0; n < NT; n++) {
+                    mma_bf16_16816(acc[n], l.x, h.x, l.y, h.y, b[i][n].x, b[i][n].y);
+                    mma_bf16_16816(acc[n], l.z, h.z, l.w, h.w, b[i][n].z, b[i][n].w);
+                }
+            }
+    }
+}
+
+// phase 1: grid (SI / 8, ceil(T / (8 * NT))); 8 warps split K; rows = 8 gate rows + the 8 matching up rows.  A ninth warp
+// produces the sigmoid gates: token i of the tile belongs to the CTA with blockIdx.x = i % gridDim.x (the first CTA
+// used to do all of them, after its rows, and every other CTA waited for it).
 template <int NT>
-__device__ __forceinline__ void warp_rows_x_tokens(const __nv_bfloat16* __restrict__ w_lo,
-                                                   const __nv_bfloat16* __restrict__ w_hi,
-                                                   const __nv_bfloat16* __restrict__ x, int ldx, int tok0, int tokens,
-                                                   int k_begin, int k_end, int lane, float (&acc)[NT][4],
-                                                   bool init = true) {
+__global__ void __launch_bounds__(288)
+shared_phase1_mma_kernel(const __nv_bfloat16* __restrict__ x, int tokens, int H, int SI,
+                         const __nv_bfloat16* __restrict__ gate_up, const __nv_bfloat16* __restrict__ shared_gate,
+                         __nv_bfloat16* __restrict__ ic2b, float* __restrict__ se_gate) {
+    constexpr int SB = NT == 8 ? 4 : 8, UB = NT == 8 ? 1 : NT == 4 ? 2 : 4;
+    __shared__ float red[8][NT][32][4];
+    pdl_launch_dependents();
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const int g8 = lane >> 2, t4 = lane & 3;
-    if (init) {
+    const int pair0 = blockIdx.x * 8, tok0 = blockIdx.y * (8 * NT);
+    if (warp < 8) {
+        const int kper = H / 8, k_end = (warp + 1) * kper;
+        const __nv_bfloat16 *w_lo = gate_up + (size_t)(pair0 + g8) * H, *w_hi = gate_up + (size_t)(SI + pair0 + g8) * H;
+        float acc[NT][4];
 #pragma unroll
         for (int n = 0; n < NT; n++)
 #pragma unroll
             for (int q = 0; q < 4; q++) acc[n][q] = 0.f;
-    }
-    const uint4 zero = make_uint4(0, 0, 0, 0);
-#pragma unroll 2
-    for (int k = k_begin + t4 * 8; k < k_end; k += 32) {
-        const uint4 alo = *reinterpret_cast<const uint4*>(w_lo + k);
-        const uint4 ahi = *reinterpret_cast<const uint4*>(w_hi + k);
+        for (int k = warp * kper + t4 * 8; k < k_end; k += SB * 32) {
+            uint4 lo[SB], hi[SB];
+            load_rows<NT, SB, UB>(lo, hi, w_lo, w_hi, k, k_end);
+            mma_rows<NT, SB, UB>(lo, hi, x, H, tok0, tokens, k, k_end, g8, acc);
+        }
 #pragma unroll
-        for (int n = 0; n < NT; n++) {
-            const int t = tok0 + n * 8 + g8;
-            const uint4 b = (t < tokens) ? *reinterpret_cast<const uint4*>(x + (size_t)t * ldx + k) : zero;
-            mma_bf16_16816(acc[n], alo.x, ahi.x, alo.y, ahi.y, b.x, b.y);
-            mma_bf16_16816(acc[n], alo.z, ahi.z, alo.w, ahi.w, b.z, b.w);
+        for (int n = 0; n < NT; n++)
+            *reinterpret_cast<float4*>(red[warp][n][lane]) = make_float4(acc[n][0], acc[n][1], acc[n][2], acc[n][3]);
+    } else {
+        for (int tl = blockIdx.x; tl < 8 * NT; tl += gridDim.x) {
+            const int t = tok0 + tl;
+            if (t >= tokens) break;
+            float a = 0.f;
+#pragma unroll 8
+            for (int k = lane * 8; k < H; k += 256) {
+                const uint4 wv = *reinterpret_cast<const uint4*>(shared_gate + k);
+                const uint4 xv = *reinterpret_cast<const uint4*>(x + (size_t)t * H + k);
+                const uint32_t ww[4] = {wv.x, wv.y, wv.z, wv.w}, xx[4] = {xv.x, xv.y, xv.z, xv.w};
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    const float2 w2 = bf16x2_to_f32(ww[q]), x2 = bf16x2_to_f32(xx[q]);
+                    a += w2.x * x2.x + w2.y * x2.y;
+                }
+            }
+            a = warp_sum(a);
+            if (lane == 0) se_gate[t] = 1.0f / (1.0f + expf(-a));
         }
     }
-}
-
-// phase 1: grid (SI / 8, ceil(T / 64)); 8 warps split K; rows = 8 gate rows + the 8 matching up rows
-__global__ void __launch_bounds__(256)
-shared_phase1_mma_kernel(const __nv_bfloat16* __restrict__ x, int tokens, int H, int SI,
-                         const __nv_bfloat16* __restrict__ gate_up, const __nv_bfloat16* __restrict__ shared_gate,
-                         __nv_bfloat16* __restrict__ ic2b, float* __restrict__ se_gate) {
-    __shared__ float red[8][kMaxTokTiles][32][4];
-    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-    const int g8 = lane >> 2, t4 = lane & 3;
-    const int pair0 = blockIdx.x * 8, tok0 = blockIdx.y * 64;
-    const int kper = H / 8;
-    float acc[kMaxTokTiles][4];
-    warp_rows_x_tokens<kMaxTokTiles>(gate_up + (size_t)(pair0 + g8) * H, gate_up + (size_t)(SI + pair0 + g8) * H, x, H,
-                                     tok0, tokens, warp * kper, (warp + 1) * kper, lane, acc);
-#pragma unroll
-    for (int n = 0; n < kMaxTokTiles; n++)
-        *reinterpret_cast<float4*>(red[warp][n][lane]) = make_float4(acc[n][0], acc[n][1], acc[n][2], acc[n][3]);
     __syncthreads();
     // warp n finishes token tile n: sum the K partials, silu(gate) * up
-    {
+    if (warp < NT) {
         const int n = warp;
         float c[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
@@ -189,52 +233,45 @@ shared_phase1_mma_kernel(const __nv_bfloat16* __restrict__ x, int tokens, int H,
             }
         }
     }
-    // the first row block also produces the sigmoid gate: one warp per token
-    if (blockIdx.x == 0) {
-        for (int tl = warp; tl < 64; tl += 8) {
-            const int t = tok0 + tl;
-            if (t >= tokens) break;
-            float a = 0.f;
-            for (int k = lane * 8; k < H; k += 256) {
-                const uint4 wv = *reinterpret_cast<const uint4*>(shared_gate + k);
-                const uint4 xv = *reinterpret_cast<const uint4*>(x + (size_t)t * H + k);
-                const uint32_t ww[4] = {wv.x, wv.y, wv.z, wv.w}, xx[4] = {xv.x, xv.y, xv.z, xv.w};
-#pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    const float2 w2 = bf16x2_to_f32(ww[q]), x2 = bf16x2_to_f32(xx[q]);
-                    a += w2.x * x2.x + w2.y * x2.y;
-                }
-            }
-            a = warp_sum(a);
-            if (lane == 0) se_gate[t] = 1.0f / (1.0f + expf(-a));
-        }
-    }
 }
 
-// phase 2: grid (H / 16, ceil(T / 64)); 2 warps split K = SI
+// phase 2: grid (H / 16, ceil(T / (8 * NT))); 2 warps split K = SI.  Launched behind phase 1 with programmatic dependent
+// launch: the weight rows (which phase 1 does not write) are asked for before its result is waited for.
+template <int NT>
 __global__ void __launch_bounds__(64)
 shared_phase2_mma_kernel(const __nv_bfloat16* __restrict__ ic2b, int tokens, int H, int SI,
                          const __nv_bfloat16* __restrict__ down, float* __restrict__ shared_out) {
-    __shared__ float red[kMaxTokTiles][32][4];
+    constexpr int SB = NT == 8 ? 4 : 8, UB = NT == 8 ? 1 : NT == 4 ? 2 : 4;
+    __shared__ float red[NT][32][4];
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const int g8 = lane >> 2, t4 = lane & 3;
-    const int d0 = blockIdx.x * 16, tok0 = blockIdx.y * 64;
-    const int kper = SI / 2;
-    float acc[kMaxTokTiles][4];
-    warp_rows_x_tokens<kMaxTokTiles>(down + (size_t)(d0 + g8) * SI, down + (size_t)(d0 + 8 + g8) * SI, ic2b, SI, tok0,
-                                     tokens, warp * kper, (warp + 1) * kper, lane, acc);
-    warp_rows_x_tokens<kMaxTokTiles>(down + (size_t)(d0 + g8) * SI, down + (size_t)(d0 + 8 + g8) * SI,
-                                     ic2b + (size_t)tokens * SI, SI, tok0, tokens, warp * kper, (warp + 1) * kper, lane,
-                                     acc, false);
+    const int d0 = blockIdx.x * 16, tok0 = blockIdx.y * (8 * NT);
+    const int kper = SI / 2, k0 = warp * kper + t4 * 8, k_end = (warp + 1) * kper;
+    const __nv_bfloat16 *w_lo = down + (size_t)(d0 + g8) * SI, *w_hi = down + (size_t)(d0 + 8 + g8) * SI;
+    float acc[NT][4];
+#pragma unroll
+    for (int n = 0; n < NT; n++)
+#pragma unroll
+        for (int q = 0; q < 4; q++) acc[n][q] = 0.f;
+    uint4 lo[SB], hi[SB];
+    load_rows<NT, SB, UB>(lo, hi, w_lo, w_hi, k0, k_end);
+    pdl_wait();
+    for (int plane = 0; plane < 2; plane++) {      // the hi plane of ic2, then the lo plane
+        const __nv_bfloat16* const xp = ic2b + (size_t)plane * tokens * SI;
+        for (int k = k0; k < k_end; k += SB * 32) {
+            if (k != k0 || (plane && kper > SB * 32)) load_rows<NT, SB, UB>(lo, hi, w_lo, w_hi, k, k_end);
+            mma_rows<NT, SB, UB>(lo, hi, xp, SI, tok0, tokens, k, k_end, g8, acc);
+        }
+    }
     if (warp == 1) {
 #pragma unroll
-        for (int n = 0; n < kMaxTokTiles; n++)
+        for (int n = 0; n < NT; n++)
             *reinterpret_cast<float4*>(red[n][lane]) = make_float4(acc[n][0], acc[n][1], acc[n][2], acc[n][3]);
     }
     __syncthreads();
     if (warp == 0) {
 #pragma unroll
-        for (int n = 0; n < kMaxTokTiles; n++) {
+        for (int n = 0; n < NT; n++) {
             const float4 v = *reinterpret_cast<const float4*>(red[n][lane]);
 #pragma unroll
             for (int q = 0; q < 2; q++) {
@@ -246,6 +283,20 @@ shared_phase2_mma_kernel(const __nv_bfloat16* __restrict__ ic2b, int tokens, int
             }
         }
     }
+}
+
+// NT: token tiles of eight per CTA
+template <int NT>
+void launch_mma(const __nv_bfloat16* x, int tokens, int H, int SI, const __nv_bfloat16* gate_up, const __nv_bfloat16* down,
+                const __nv_bfloat16* shared_gate, __nv_bfloat16* ic2b, float* shared_out, float* se_gate, const Ctx& c) {
+    const int tiles = (tokens + 8 * NT - 1) / (8 * NT);
+    c.begin(K_SHARED_PHASE1);
+    shared_phase1_mma_kernel<NT><<<dim3(SI / 8, tiles), 288, 0, c.s>>>(x, tokens, H, SI, gate_up, shared_gate, ic2b, se_gate);
+    c.end();
+    c.begin(K_SHARED_PHASE2);
+    launch_pdl(shared_phase2_mma_kernel<NT>, dim3(H / 16, tiles), dim3(64), 0, c.s, (const __nv_bfloat16*)ic2b, tokens, H, SI, down,
+               shared_out);
+    c.end();
 }
 
 }  // namespace
@@ -262,14 +313,10 @@ int launch_shared_expert(const __nv_bfloat16* x, int tokens, int hidden, int sha
     // tensor-core path: K splits must be multiples of 32
     if (hidden % 256 == 0 && shared_inter % 64 == 0 && hidden % 16 == 0 && shared_inter % 8 == 0) {
         __nv_bfloat16* ic2b = reinterpret_cast<__nv_bfloat16*>(ic2s);
-        dim3 g1(shared_inter / 8, (tokens + 63) / 64);
-        c.begin(K_SHARED_PHASE1);
-        shared_phase1_mma_kernel<<<g1, 256, 0, c.s>>>(x, tokens, hidden, shared_inter, gate_up, shared_gate, ic2b, se_gate);
-        c.end();
-        dim3 g2(hidden / 16, (tokens + 63) / 64);
-        c.begin(K_SHARED_PHASE2);
-        shared_phase2_mma_kernel<<<g2, 64, 0, c.s>>>(ic2b, tokens, hidden, shared_inter, down, shared_out);
-        c.end();
+        // up to 8, 16, 32 and 64 tokens per CTA: the tiles a small batch does not fill cost MMAs and registers, and a
+        // weight row is read once per CTA
+        auto* const launch = tokens <= 8 ? launch_mma<1> : tokens <= 16 ? launch_mma<2> : tokens <= 32 ? launch_mma<4> : launch_mma<8>;
+        launch(x, tokens, hidden, shared_inter, gate_up, down, shared_gate, ic2b, shared_out, se_gate, c);
         return 2;
     }
     const int ttiles = (tokens + kTokTile - 1) / kTokTile;
