@@ -247,6 +247,7 @@ static_assert(kTmWBoxBytes % 128 == 0 && kTmSBoxBytes % 128 == 0, "TMA destinati
 
 struct DenseMaps {
     CUtensorMap packed, scale;
+    CUtensorMap x;      // bf16 activations (tensor-memory kernel)
 };
 
 template <int NT>
@@ -429,9 +430,9 @@ void launch_tma(const DenseMaps& maps, const DenseArgs& a, int sm_count, cudaStr
     dense_gemv_tma_kernel<NT><<<sm_count, (kTmWarps + 1) * 32, tma_smem<NT>(a.K), s>>>(maps, a);
 }
 
-// [rows, inner] matrix of `esize`-byte elements, row-major, box = box_inner x box_rows, no swizzle
+// [rows, inner] matrix of `esize`-byte elements, row-major, box = box_inner x box_rows
 bool make_plain_map(CUtensorMap* map, CUtensorMapDataType type, int esize, const void* base, size_t inner, size_t rows,
-                    int box_inner, int box_rows) {
+                    int box_inner, int box_rows, CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_NONE) {
     umma::EncodeTiledFn fn = umma::encode_tiled();
     if (!fn) return false;
     cuuint64_t dims[2] = {(cuuint64_t)inner, (cuuint64_t)rows};
@@ -439,7 +440,362 @@ bool make_plain_map(CUtensorMap* map, CUtensorMapDataType type, int esize, const
     cuuint32_t box[2] = {(cuuint32_t)box_inner, (cuuint32_t)box_rows};
     cuuint32_t estr[2] = {1, 1};
     return fn(map, type, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-              CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+              swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// ---- the same product on the 5th-generation tensor cores, for more than kUmmaMinTok tokens ------------
+// The kernels above serve sixteen tokens per pass over the bank and are bound by their conversions and the
+// mma.sync rate from there on (95 us a pass at 248 320 x 2048), so 64 tokens were four passes (408 us).  Here one pass
+// serves up to 64: the dequantised weights are the A operand in tensor memory (one lane per weight row, as in the
+// grouped GEMM of prefill_umma.cu), the tokens are the B operand in shared memory, f32 accumulators in tensor memory.
+// Unit = 256 rows (two tiles of 128) x the whole of K, persistent CTAs of 24 warps:
+//   warp 0        TMA: [32 k-words x 128 rows] packed words and [16 blocks x 128 rows] block scales into a raw ring.
+//                 The bank is K-major, so a k-word of a tile is one 512-byte run and lane = row reads it without
+//                 bank conflicts
+//   warps 1, 3    tcgen05.mma issuers, one per row tile (M = 128, N = tokens rounded up to 16)
+//   warp 2        TMA: tiles of 64 tokens x 64 k of bf16 activations (they stay in L2), 128-byte swizzle
+//   warps 4..7    rewrite every such tile in place as f16, scaled per token by a power of two (exact).  Converting the
+//                 activations again for every unit costs these four warps less time than the unit takes, and needs
+//                 no scratch buffer that calls on two streams would share.  f32 activations they read themselves
+//   warps 8..15   two dequantiser sets, two weight buffers each
+//   warps 16..23  epilogue, one set per row tile: sums the accumulators, applies token scale and row global,
+//                 stores whole rows (no K split: nothing to clear, no atomics)
+// Consecutive 64-k steps go to different accumulators in turn (two for 64 tokens, four for 32), summed in f32 by the
+// epilogue: the chain of one accumulator stays short, as in the kernels above.
+// Every mbarrier wait is bounded; a wait that gives up raises the error flag and the CTA drains.
+constexpr int kUmmaMinTok = 16;   // sixteen tokens are one pass of either kernel: 97.8 us above, 101.6 us here
+constexpr int kUmThreads = 768;
+constexpr int kUmTok = 64;                     // most tokens per pass
+constexpr int kUmXStages = 8, kUmRawStages = 6;
+constexpr int kUmXBytes = kUmTok * 128;        // 64 tokens x 64 k f16
+constexpr int kUmPackedBytes = 32 * 128 * 4, kUmScaleBytes = 16 * 128;
+constexpr int kUmRawBytes = kUmPackedBytes + kUmScaleBytes;
+constexpr int kUmWBufs = 4, kUmWCols = 64;     // dequantised chunks of 128 k in tensor memory
+constexpr int kUmAccCol0 = kUmWBufs * kUmWCols, kUmAccCols = 128;   // accumulator columns of one row tile
+constexpr size_t kUmSmem = 1024 + (size_t)kUmXStages * kUmXBytes + (size_t)kUmRawStages * kUmRawBytes + 48 * 8 + kUmTok * 4 + 64;
+
+template <bool F32>
+__global__ void __launch_bounds__(kUmThreads, 1)
+dense_gemv_umma_kernel(const __grid_constant__ DenseMaps maps, DenseArgs a) {
+    using namespace umma;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* const smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    uint8_t* const x_tiles = smem;
+    uint8_t* const raw_ring = smem + kUmXStages * kUmXBytes;
+    uint64_t* const bars = reinterpret_cast<uint64_t*>(raw_ring + kUmRawStages * kUmRawBytes);
+    float* const s_scale = reinterpret_cast<float*>(bars + 48);     // per token: the power of two its row was divided by
+    uint32_t* const s_tmem = reinterpret_cast<uint32_t*>(s_scale + kUmTok);
+    volatile int* const s_abort = reinterpret_cast<volatile int*>(s_tmem + 1);
+    const uint32_t bar0 = smem_u32(bars);
+    auto X_FULL = [&](int s) { return bar0 + 8u * s; };
+    auto X_EMPTY = [&](int s) { return bar0 + 8u * (8 + s); };
+    auto RAW_FULL = [&](int s) { return bar0 + 8u * (16 + s); };
+    auto RAW_EMPTY = [&](int s) { return bar0 + 8u * (22 + s); };
+    auto W_READY = [&](int s) { return bar0 + 8u * (28 + s); };
+    auto W_FREE = [&](int s) { return bar0 + 8u * (32 + s); };
+    const uint32_t ACC_FULL = bar0 + 8u * 36, ACC_EMPTY = bar0 + 8u * 37;
+    auto XRAW_FULL = [&](int s) { return bar0 + 8u * (38 + s); };
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < kUmXStages; s++) {
+            mbar_init(XRAW_FULL(s), 1);
+            mbar_init(X_FULL(s), 128);
+            mbar_init(X_EMPTY(s), 2);
+        }
+        for (int s = 0; s < kUmRawStages; s++) {
+            mbar_init(RAW_FULL(s), 1);
+            mbar_init(RAW_EMPTY(s), 256);
+        }
+        for (int s = 0; s < kUmWBufs; s++) {
+            mbar_init(W_READY(s), 128);
+            mbar_init(W_FREE(s), 1);
+        }
+        mbar_init(ACC_FULL, 2);
+        mbar_init(ACC_EMPTY, 256);
+        *s_abort = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(s_tmem)) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem_base = *s_tmem;
+
+    const int K = a.K, N = a.N;
+    const int chunks = K / 128, items_per_unit = 2 * chunks;    // (chunk, row tile) pieces; chunks is even
+    const int n_units = (N + 255) / 256;
+    const int n_pad = (a.ntok + 15) & ~15;
+    const int splits = n_pad <= 32 ? 4 : 2, acc_stride = kUmAccCols / splits;
+
+    if (warp != 0) {
+        // the power of two of every token (the weight producer is already at work): largest magnitude into [2^14, 2^15)
+        for (int tk = warp - 1; tk < a.ntok; tk += kUmThreads / 32 - 1) {
+            const size_t row = (size_t)(a.tok0 + tk) * K;
+            float m = 0.f;
+#pragma unroll 8
+            for (int k = lane * (F32 ? 4 : 8); k < K; k += F32 ? 128 : 256) {
+                if (F32) {
+                    const float4 v = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(a.a) + row + k);
+                    m = fmaxf(fmaxf(fmaxf(m, fabsf(v.x)), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
+                } else {
+                    const uint4 u = *reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(a.a) + row + k);
+                    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+                    for (int q = 0; q < 4; q++) {
+                        const float2 f = bf16x2_to_f32(w[q]);
+                        m = fmaxf(m, fmaxf(fabsf(f.x), fabsf(f.y)));
+                    }
+                }
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+            // (exponents below 15 would need a factor past the largest float: such rows keep 15's, exact all the same)
+            const int e = max((int)((__float_as_uint(m) >> 23) & 0xff), 15);
+            if (lane == 0) s_scale[tk] = e < 255 ? __uint_as_float((uint32_t)(127 - 14 + (e - 127)) << 23) : 1.0f;
+        }
+        asm volatile("bar.sync 1, %0;" ::"n"(kUmThreads - 32) : "memory");
+    }
+
+    if (warp == 0) {
+        // ===================== packed weights and block scales =======================================
+        uint32_t it = 0;
+        for (int u = blockIdx.x; u < n_units && !*s_abort; u += gridDim.x) {
+            bool ok = true;
+            for (int q = 0; q < chunks && ok; q++, it++) {     // a stage = two chunks (256 k) of one row tile
+                const int cp = q >> 1, r = q & 1, st = it % kUmRawStages;
+                ok = mbar_wait_warp(RAW_EMPTY(st), ((it / kUmRawStages) & 1) ^ 1, s_abort, a.err);
+                if (!ok) break;
+                if (elect_one()) {
+                    const uint32_t dst = smem_u32(raw_ring + (size_t)st * kUmRawBytes);
+                    mbar_expect_tx(RAW_FULL(st), kUmRawBytes);      // rows past N read as zero and count like the others
+                    tma_load_2d(dst, &maps.packed, u * 256 + r * 128, cp * 32, RAW_FULL(st));
+                    tma_load_2d(dst + kUmPackedBytes, &maps.scale, u * 256 + r * 128, cp * 16, RAW_FULL(st));
+                }
+                __syncwarp();
+            }
+            if (!ok) break;
+        }
+    } else if (warp == 2) {
+        // ===================== bf16 activation tiles ================================================
+        if constexpr (!F32) {
+            uint32_t it = 0;
+            for (int u = blockIdx.x; u < n_units && !*s_abort; u += gridDim.x) {
+                bool ok = true;
+                for (int ks = 0; ks < K / 64; ks++, it++) {
+                    const int st = it % kUmXStages;
+                    ok = mbar_wait_warp(X_EMPTY(st), ((it / kUmXStages) & 1) ^ 1, s_abort, a.err);
+                    if (!ok) break;
+                    if (elect_one()) {
+                        mbar_expect_tx(XRAW_FULL(st), kUmXBytes);      // rows past the last token read as zero
+                        tma_load_2d(smem_u32(x_tiles + (size_t)st * kUmXBytes), &maps.x, ks * 64, a.tok0, XRAW_FULL(st));
+                    }
+                    __syncwarp();
+                }
+                if (!ok) break;
+            }
+        }
+    } else if (warp == 1 || warp == 3) {
+        // ===================== MMA issuers (see the grouped GEMM for the looks ahead) ================
+        const int r = warp >> 1;
+        const uint32_t idesc = (1u << 4) | ((uint32_t)(128 >> 4) << 24) | ((uint32_t)(n_pad >> 3) << 17);
+        const uint32_t d_tmem = tmem_base + kUmAccCol0 + r * kUmAccCols;
+        uint32_t it = 0, item = r, unit_i = 0;
+        bool x_seen = false, w_seen = false;
+        for (int u = blockIdx.x; u < n_units && !*s_abort; u += gridDim.x, unit_i++) {
+            bool ok = mbar_wait_warp(ACC_EMPTY, (unit_i & 1) ^ 1, s_abort, a.err);
+            for (int ks = 0; ks < 2 * chunks && ok; ks++, it++) {
+                const int h = ks & 1, wb = item % kUmWBufs, st = it % kUmXStages;
+                if (h == 0 && !w_seen) ok = mbar_wait_warp(W_READY(wb), (item / kUmWBufs) & 1, s_abort, a.err);
+                if (!ok) break;
+                if (!x_seen) ok = mbar_wait_warp(X_FULL(st), (it / kUmXStages) & 1, s_abort, a.err);
+                if (!ok) break;
+                {
+                    const uint32_t it1 = it + 1;
+                    x_seen = __all_sync(0xffffffffu, mbar_test_wait(X_FULL(it1 % kUmXStages), (it1 / kUmXStages) & 1));
+                    if (h == 1) {
+                        const uint32_t item1 = item + 2;
+                        w_seen = __all_sync(0xffffffffu, mbar_test_wait(W_READY(item1 % kUmWBufs), (item1 / kUmWBufs) & 1));
+                    }
+                }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t w_addr = tmem_base + wb * kUmWCols;
+                const uint64_t xdesc = umma_desc(smem_u32(x_tiles + (size_t)st * kUmXBytes));
+                const uint32_t d = d_tmem + (ks & (splits - 1)) * acc_stride;
+                if (elect_one()) {
+#pragma unroll
+                    for (int kk = 0; kk < 4; kk++)
+                        umma_f16_ts(d, w_addr + (h * 4 + kk) * 8, xdesc + kk * 2, idesc, (ks >= splits || kk > 0) ? 1u : 0u);
+                    umma_commit(X_EMPTY(st));
+                    if (h == 1) umma_commit(W_FREE(wb));
+                }
+                __syncwarp();
+                if (h == 1) item += 2;
+            }
+            if (!ok) break;
+            if (elect_one()) umma_commit(ACC_FULL);
+            __syncwarp();
+        }
+    } else if (warp >= 4 && warp < 8) {
+        // ===================== activations: two threads per token, 32 k each ==========================
+        const int tid = threadIdx.x - 128, tok = tid >> 1, half = tid & 1;
+        const bool live = tok < a.ntok, in_tile = tok < n_pad;      // (a row past this pass's may be another's: its factor is 0)
+        const int steps = K / 64;
+        const float inv = live ? 1.0f / s_scale[tok] : 0.f;       // a power of two: exact
+        const float* const src = reinterpret_cast<const float*>(a.a) + (size_t)(a.tok0 + (live ? tok : 0)) * K + half * 32;
+        float4 buf[F32 ? 8 : 1];      // f32: the next step's 32 k, loaded a step ahead
+        auto load = [&](int ks) {
+#pragma unroll
+            for (int v = 0; v < 8; v++)
+                buf[v] = live ? *reinterpret_cast<const float4*>(src + (size_t)ks * 64 + v * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+        };
+        uint32_t it = 0;
+        for (int u = blockIdx.x; u < n_units && !*s_abort; u += gridDim.x) {
+            bool ok = true;
+            if constexpr (F32) load(0);
+            for (int ks = 0; ks < steps; ks++, it++) {
+                const int st = it % kUmXStages;
+                uint8_t* const row = x_tiles + (size_t)st * kUmXBytes + tok * 128;
+                __half2 h2[16];
+                if constexpr (F32) {
+#pragma unroll
+                    for (int v = 0; v < 8; v++) {
+                        h2[2 * v] = __floats2half2_rn(buf[v].x * inv, buf[v].y * inv);
+                        h2[2 * v + 1] = __floats2half2_rn(buf[v].z * inv, buf[v].w * inv);
+                    }
+                    if (ks + 1 < steps) load(ks + 1);
+                    ok = mbar_wait(X_EMPTY(st), ((it / kUmXStages) & 1) ^ 1, s_abort, a.err);
+                    if (!ok) break;
+                } else {
+                    ok = mbar_wait(XRAW_FULL(st), (it / kUmXStages) & 1, s_abort, a.err);
+                    if (!ok) break;
+                    if (in_tile) {
+#pragma unroll
+                        for (int j = 0; j < 4; j++) {
+                            const uint4 v = *reinterpret_cast<const uint4*>(row + (((half * 4 + j) ^ (tok & 7)) << 4));
+                            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                            for (int q = 0; q < 4; q++) {
+                                const float2 f = bf16x2_to_f32(w[q]);
+                                h2[4 * j + q] = __floats2half2_rn(f.x * inv, f.y * inv);
+                            }
+                        }
+                    }
+                }
+                if (in_tile) {
+#pragma unroll
+                    for (int j = 0; j < 4; j++)
+                        *reinterpret_cast<uint4*>(row + (((half * 4 + j) ^ (tok & 7)) << 4)) =
+                            make_uint4(*reinterpret_cast<uint32_t*>(&h2[4 * j]), *reinterpret_cast<uint32_t*>(&h2[4 * j + 1]),
+                                       *reinterpret_cast<uint32_t*>(&h2[4 * j + 2]), *reinterpret_cast<uint32_t*>(&h2[4 * j + 3]));
+                }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");     // the tensor core reads what this thread stored
+                mbar_arrive(X_FULL(st));
+            }
+            if (!ok) break;
+        }
+    } else if (warp >= 8 && warp < 16) {
+        // ===================== dequantisers: raw ring -> f16 weights in tensor memory ================
+        const int quarter = warp & 3, set = (warp - 8) >> 2;
+        const int row = quarter * 32 + lane;
+        const uint32_t tlane = tmem_base + ((uint32_t)(quarter * 32) << 16);
+        uint32_t item0 = 0, stage0 = 0;
+        for (int u = blockIdx.x; u < n_units && !*s_abort; u += gridDim.x, item0 += items_per_unit, stage0 += chunks) {
+            bool ok = true;
+            for (int w = set; w < items_per_unit; w += 2) {
+                const uint32_t item = item0 + w;
+                const int c = w >> 1;
+                const uint32_t stage = stage0 + 2 * (c >> 1) + (w & 1);
+                const int st = stage % kUmRawStages;
+                ok = mbar_wait(RAW_FULL(st), (stage / kUmRawStages) & 1, s_abort, a.err);
+                if (!ok) break;
+                const int wb = item % kUmWBufs;
+                const uint32_t taddr = tlane + wb * kUmWCols;
+                const uint8_t* const rp = raw_ring + (size_t)st * kUmRawBytes + (c & 1) * 16 * 512 + row * 4;
+                const uint8_t* const sp = raw_ring + (size_t)st * kUmRawBytes + kUmPackedBytes + (c & 1) * 8 * 128 + row;
+                // 32 k (four k-words, two block scales) -> 16 columns
+                auto convert = [&](int g, uint32_t (&r)[16]) {
+                    const uint32_t two = (uint32_t)sp[(2 * g) * 128] | ((uint32_t)sp[(2 * g + 1) * 128] << 8);
+                    uint32_t h2;
+                    asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(h2) : "h"((uint16_t)two));
+                    const uint32_t s0 = __byte_perm(h2, h2, 0x1010), s1 = __byte_perm(h2, h2, 0x3232);
+#pragma unroll
+                    for (int j = 0; j < 4; j++) {
+                        uint32_t q[4];
+                        e2m1x8_to_f16x2(*reinterpret_cast<const uint32_t*>(rp + (4 * g + j) * 512), q);
+#pragma unroll
+                        for (int e = 0; e < 4; e++) r[4 * j + e] = hmul2_f16(q[e], (j < 2) ? s0 : s1);
+                    }
+                };
+                uint32_t r0[16], r1[16];
+                convert(0, r0);
+                convert(1, r1);
+                ok = mbar_wait(W_FREE(wb), ((item / kUmWBufs) & 1) ^ 1, s_abort, a.err);
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                tmem_st16(taddr, r0);
+                tmem_st16(taddr + 16, r1);
+                convert(2, r0);
+                tmem_st16(taddr + 32, r0);
+                convert(3, r1);
+                tmem_st16(taddr + 48, r1);
+                mbar_arrive(RAW_EMPTY(st));
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                mbar_arrive(W_READY(wb));
+            }
+            if (!ok) break;
+        }
+    } else if (warp >= 16) {
+        // ===================== epilogue: one thread = one weight row, a column = one token =============
+        const int quarter = warp & 3, r = (warp - 16) >> 2;
+        uint32_t unit_i = 0;
+        for (int u = blockIdx.x; u < n_units && !*s_abort; u += gridDim.x, unit_i++) {
+            const int n = u * 256 + r * 128 + quarter * 32 + lane;
+            const float gl = n < N ? f16_global_to_f32(a.global[n]) : 0.f;
+            if (!mbar_wait(ACC_FULL, unit_i & 1, s_abort, a.err)) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + kUmAccCol0 + r * kUmAccCols;
+#pragma unroll 1
+            for (int c0 = 0; c0 < a.ntok; c0 += 16) {
+                float v[16], v1[16];
+                tmem_ld16(taddr + c0, v);
+                tmem_ld16(taddr + acc_stride + c0, v1);
+                tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < 16; j++) v[j] += v1[j];
+                if (splits == 4) {
+                    float v2[16];
+                    tmem_ld16(taddr + 2 * acc_stride + c0, v1);
+                    tmem_ld16(taddr + 3 * acc_stride + c0, v2);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 16; j++) v[j] += v1[j] + v2[j];
+                }
+                if (n < N) {
+                    float* const dst = a.c + (size_t)(a.tok0 + c0) * N + n;
+#pragma unroll
+                    for (int j = 0; j < 16; j++)
+                        if (c0 + j < a.ntok) dst[(size_t)j * N] = (v[j] * s_scale[c0 + j]) * gl;
+                }
+                __syncwarp();
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            mbar_arrive(ACC_EMPTY);
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem_base) : "memory");
+}
+
+template <bool F32>
+void launch_umma(const DenseMaps& maps, const DenseArgs& a, int sm_count, cudaStream_t s) {
+    static PerDeviceOnce once;
+    allow_dyn_smem(once, dense_gemv_umma_kernel<F32>, kUmSmem);
+    dense_gemv_umma_kernel<F32><<<sm_count, kUmThreads, kUmSmem, s>>>(maps, a);
 }
 
 template <int NT>
@@ -469,11 +825,31 @@ int launch_dense_gemv(const void* a, int a_dtype, const uint32_t* packed, const 
                      make_plain_map(&maps.packed, CU_TENSOR_MAP_DATA_TYPE_INT32, 4, packed, (size_t)N, (size_t)K / 8, kTmBoxRows, kTmKw) &&
                      make_plain_map(&maps.scale, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, scale, (size_t)N, (size_t)K / 16, kTmUseRows, kTmKw / 2);
     d.splits = (tma || K % 64 == 0) ? 2 : 1;
-    int launches = 0;
-    if (d.splits > 1) cudaMemsetAsync(c, 0, (size_t)M * N * sizeof(float), ctx.s);
+    // More tokens than one pass of the kernels above serves: the tensor-memory kernel, under their alignment rules for
+    // the bank (its units are 256 rows) and with activations that can be read 16 bytes at a time.  A remainder of up to
+    // kUmmaMinTok tokens after passes of 64 goes to the kernels above.
+    DenseMaps umaps;
+    const bool umma = M > kUmmaMinTok && N % 16 == 0 && K % 256 == 0 && N >= 256 && (reinterpret_cast<uintptr_t>(packed) & 15) == 0 &&
+                      (reinterpret_cast<uintptr_t>(scale) & 15) == 0 && (reinterpret_cast<uintptr_t>(a) & 15) == 0 &&
+                      make_plain_map(&umaps.packed, CU_TENSOR_MAP_DATA_TYPE_INT32, 4, packed, (size_t)N, (size_t)K / 8, 128, 32) &&
+                      make_plain_map(&umaps.scale, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, scale, (size_t)N, (size_t)K / 16, 128, 16) &&
+                      (a_dtype == 1 || make_plain_map(&umaps.x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, a, (size_t)K, (size_t)M, 64, kUmTok,
+                                                      CU_TENSOR_MAP_SWIZZLE_128B));
+    int launches = 0, t0 = 0;
     ctx.begin(K_DENSE_GEMV);
+    for (; umma && M - t0 > kUmmaMinTok; t0 += kUmTok) {
+        d.tok0 = t0;
+        d.ntok = (M - t0 < kUmTok) ? M - t0 : kUmTok;
+        if (a_dtype == 1)
+            launch_umma<true>(umaps, d, sm_count, ctx.s);
+        else
+            launch_umma<false>(umaps, d, sm_count, ctx.s);
+        launches++;
+    }
+    // the K halves of the kernels above add into c
+    if (t0 < M && d.splits > 1) cudaMemsetAsync(c + (size_t)t0 * N, 0, (size_t)(M - t0) * N * sizeof(float), ctx.s);
     // sixteen tokens per pass over the weights (the decode tail runs at one token per sequence)
-    for (int t0 = 0; t0 < M; t0 += 16) {
+    for (; t0 < M; t0 += 16) {
         d.tok0 = t0;
         d.ntok = (M - t0 < 16) ? M - t0 : 16;
         if (tma) {

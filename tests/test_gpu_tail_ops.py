@@ -226,6 +226,34 @@ def test_dense_gemv_lm_head_size(m):
     moe.close()
 
 
+@pytest.mark.parametrize("dtype", ["bf16", "f32"])
+@pytest.mark.parametrize("m,n,k", [(17, 272, 256), (31, 256, 512), (32, 528, 768), (33, 1040, 2048), (48, 4112, 2048),
+                                   (63, 384, 2048), (64, 65552, 256), (65, 272, 512), (81, 512, 256), (130, 304, 768)])
+def test_dense_gemv_many_tokens_against_cpu_path(m, n, k, dtype):
+    """More than sixteen tokens with N % 16 == 0, K % 256 == 0: the tensor-memory kernel.  Token counts either side of its
+    16-token and 32-token steps and of the 64 of one pass (a remainder of one goes to the other kernel, 17 and more
+    to a second pass), a last unit of 16 rows, one without its second tile, more units than SMs, two to sixteen chunks
+    of K.  f32 activations keep eleven bits each (half an ulp: 2^-12 relative), independent errors over K products, so
+    the row error stays below 2^-12; bf16 activations are exact."""
+    a, pk, sk, glob = _gemv_case(m, n, k, 77 + m + n + k)
+    x = o.bf16_bits_to_f32(a).copy()
+    if dtype == "f32":
+        x *= 1.0 + np.random.default_rng(m).uniform(0, 2.0 ** -8, x.shape).astype(np.float32)
+    x[m // 2] *= 2.0 ** -20          # rows of very different size, one of zeros
+    x[m - 1] = 0.0
+    moe = tiny_handle(64)
+    t = torch.from_numpy(x).to(dev())
+    c = moe.dense_gemv(t if dtype == "f32" else t.to(torch.bfloat16), torch.from_numpy(pk.view(np.int32)).to(dev()),
+                       torch.from_numpy(sk).to(dev()), torch.from_numpy(glob.view(np.int16)).to(dev()))
+    moe.sync_status()
+    got = c.cpu().numpy()
+    want = o.nvfp4_dense_gemv(x, pk, sk, glob.view(np.uint16))
+    tol = 1e-5 if dtype == "bf16" else 2.0 ** -12
+    for i in range(m):
+        assert np.linalg.norm(got[i] - want[i]) <= tol * np.linalg.norm(want[i]), i
+    moe.close()
+
+
 def test_dense_gemv_rejects_shapes_it_was_not_built_for():
     moe = tiny_handle(64)
     a, pk, sk, glob = _gemv_case(1, 8, 64, 5)
