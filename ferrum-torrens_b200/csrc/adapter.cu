@@ -607,7 +607,7 @@ static int router_locked(ftm_handle* h, const void* x, const void* gate_w, int32
                                            h->cfg.top_k, ids_out, weights_out, h->ctx(s));
     } else {
         h->launches += launch_router_logits((const __nv_bfloat16*)x, (const __nv_bfloat16*)gate_w, tokens, h->cfg.experts,
-                                            h->cfg.hidden, h->logits, h->ctx(s));
+                                            h->cfg.hidden, h->logits, h->sm_total, h->ctx(s));
         h->launches += launch_router_topk(h->logits, tokens, h->cfg.experts, h->cfg.top_k, ids_out, weights_out, h->ctx(s));
     }
     CU(h, cudaGetLastError());

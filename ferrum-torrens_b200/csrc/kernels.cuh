@@ -86,7 +86,7 @@ inline cudaError_t allow_dyn_smem(PerDeviceOnce& once, KernelT kernel, size_t by
 
 // router.cu
 int launch_router_logits(const __nv_bfloat16* x, const __nv_bfloat16* gate_w, int tokens, int experts,
-                         int hidden, float* logits, const Ctx& c);
+                         int hidden, float* logits, int sm_count, const Ctx& c);
 int launch_router_topk(const float* logits, int tokens, int experts, int top_k, int32_t* ids,
                        float* weights, const Ctx& c);
 

@@ -87,61 +87,66 @@ router_logits_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* _
     }
 }
 
-// ---- tiled variant for hidden % 256 == 0 -----------------------------------------------------
-// CTA = 4 warps, tile = 32 experts x 16 tokens; lane = expert, each warp owns 4 tokens, so a thread
-// walks 4 independent chains (enough to cover the FMA latency).  The gate rows stream through a
-// double-buffered shared tile filled with 16-byte cp.async; the activations are widened to f32
-// and stored k-major so that one broadcast 128-bit load feeds the warp's 4 tokens.
-constexpr int kTileE = 32, kTileT = 16, kKC = 256;
-constexpr int kWStride = kKC * 2 + 16;  // bytes per expert row in shared memory (conflict-free 128-bit reads)
-
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 
-__global__ void __launch_bounds__(128)
-router_logits_tiled_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gate_w,
-                           int tokens, int experts, int hidden, float* __restrict__ logits) {
+// ---- narrow variant for hidden % 256 == 0 ----------------------------------------------------
+// CTA = 4 warps, tile = 32 * NE experts x 16 tokens; a lane owns experts lane (and lane + 32), a warp 4 tokens: 4 or 8
+// chains per thread.  The gate rows stream through a double-buffered shared tile filled with 16-byte cp.async; the activations are
+// widened to f32 and stored k-major so that one broadcast 128-bit load feeds the warp's 4 tokens.  What bounds it is the
+// shared-memory pipe (a broadcast 128-bit load costs two of its cycles, a row load eight) and the FMA latency of few
+// warps: with one expert per lane the activations are loaded twice as often (logits + top-k at 512 tokens 42.5 us, with
+// two 31.5); one expert per lane is for the batches whose 32-expert tiles are at most one per SM (256 tokens 25.6 us, with two 31.3).  Packing two chains into fma.rn.f32x2 brought nothing: it issues at less than half the rate of the scalar fma.
+constexpr int kNT = 4, kNK = 128;
+constexpr int kNTok = 4 * kNT;
+constexpr int kNWStride = kNK * 2 + 16;     // bytes per expert row in shared memory (conflict-free 128-bit reads)
+
+template <int kNE>
+__global__ void __launch_bounds__(128, 3)
+router_logits_narrow_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gate_w,
+                            int tokens, int experts, int hidden, float* __restrict__ logits) {
+    constexpr int kNExp = 32 * kNE;
     extern __shared__ __align__(16) uint8_t rsm[];
-    uint8_t* const wbuf = rsm;                                                  // [2][32][kWStride]
-    float* const xbuf = reinterpret_cast<float*>(rsm + 2 * kTileE * kWStride);  // [2][kKC][16]
+    uint8_t* const wbuf = rsm;                                                  // [2][kNExp][kNWStride]
+    float* const xbuf = reinterpret_cast<float*>(rsm + 2 * kNExp * kNWStride);  // [2][kNK][kNTok]
     const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
-    const int e0 = blockIdx.x * kTileE, t0 = blockIdx.y * kTileT;
-    const int nchunks = hidden / kKC;
+    const int e0 = blockIdx.x * kNExp, t0 = blockIdx.y * kNTok;
+    const int nchunks = hidden / kNK;
     const uint32_t wbase = (uint32_t)__cvta_generic_to_shared(wbuf);
 
     auto issue_w = [&](int c, int b) {
-        for (int i = tid; i < kTileE * (kKC / 8); i += 128) {
-            const int row = i / (kKC / 8), piece = i % (kKC / 8);
+#pragma unroll 4
+        for (int i = tid; i < kNExp * (kNK / 8); i += 128) {
+            const int row = i / (kNK / 8), piece = i % (kNK / 8);
             const int e = min(e0 + row, experts - 1);
-            cp_async16(wbase + b * kTileE * kWStride + row * kWStride + piece * 16,
-                       gate_w + (size_t)e * hidden + c * kKC + piece * 8);
+            cp_async16(wbase + b * kNExp * kNWStride + row * kNWStride + piece * 16, gate_w + (size_t)e * hidden + c * kNK + piece * 8);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    // activations: thread -> token tid % 16, 16-byte pieces tid / 16 + 8 * i
-    const int xtl = tid % 16, xpc = tid / 16;
-    uint4 xr[4];
+    // activations: thread -> token tid % 16, every eighth 16-byte piece of the chunk
+    constexpr int kXStep = 128 / kNTok, kXPieces = kNK / 8 / kXStep;
+    const int xtl = tid % kNTok, xpc = tid / kNTok;
+    uint4 xr[kXPieces];
     auto load_x = [&](int c) {
         const int t = t0 + xtl;
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
+        for (int i = 0; i < kXPieces; i++) {
             xr[i] = make_uint4(0, 0, 0, 0);
-            if (t < tokens)
-                xr[i] = *reinterpret_cast<const uint4*>(x + (size_t)t * hidden + c * kKC + (xpc + 8 * i) * 8);
+            if (t < tokens) xr[i] = *reinterpret_cast<const uint4*>(x + (size_t)t * hidden + c * kNK + (xpc + kXStep * i) * 8);
         }
     };
     auto store_x = [&](int b) {
-        float* xs = xbuf + b * kKC * kTileT;
+        float* xs = xbuf + b * kNK * kNTok;
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const int k = (xpc + 8 * i) * 8;
+        for (int i = 0; i < kXPieces; i++) {
+            const int k = (xpc + kXStep * i) * 8;
             const uint32_t w[4] = {xr[i].x, xr[i].y, xr[i].z, xr[i].w};
 #pragma unroll
             for (int q = 0; q < 4; q++) {
                 const float2 v = bf16x2_to_f32(w[q]);
-                xs[(k + 2 * q) * kTileT + xtl] = v.x;
-                xs[(k + 2 * q + 1) * kTileT + xtl] = v.y;
+                xs[(k + 2 * q) * kNTok + xtl] = v.x;
+                xs[(k + 2 * q + 1) * kNTok + xtl] = v.y;
             }
         }
     };
@@ -149,8 +154,11 @@ router_logits_tiled_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloa
     issue_w(0, 0);
     load_x(0);
     store_x(0);
-    const bool active = t0 + warp * 4 < tokens;
-    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+    float acc[kNE][kNT];
+#pragma unroll
+    for (int j = 0; j < kNE; j++)
+#pragma unroll
+        for (int i = 0; i < kNT; i++) acc[j][i] = 0.f;
     for (int c = 0; c < nchunks; c++) {
         const int b = c & 1;
         asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -159,54 +167,37 @@ router_logits_tiled_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloa
             issue_w(c + 1, b ^ 1);
             load_x(c + 1);
         }
-        if (active) {
-            const uint32_t wrow = wbase + b * kTileE * kWStride + lane * kWStride;
-            const float* xs = xbuf + b * kKC * kTileT + warp * 4;
-            // operands of the next eight k are fetched while the current eight are multiplied
-            uint4 wc;
-            float4 xc[8];
-            auto fetch = [&](int kk, uint4& wv, float4 (&xv)[8]) {
-                asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
-                             : "=r"(wv.x), "=r"(wv.y), "=r"(wv.z), "=r"(wv.w)
-                             : "r"(wrow + kk * 2));
-#pragma unroll
-                for (int q = 0; q < 8; q++) xv[q] = *reinterpret_cast<const float4*>(xs + (kk + q) * kTileT);
-            };
-            fetch(0, wc, xc);
+        const uint8_t* const wrow = wbuf + b * kNExp * kNWStride + lane * kNWStride;
+        const float* const xs = xbuf + b * kNK * kNTok + warp * kNT;
 #pragma unroll 2
-            for (int kk = 0; kk < kKC; kk += 8) {
-                uint4 wn = wc;
-                float4 xn[8];
+        for (int kk = 0; kk < kNK; kk += 8) {
+            uint4 wq[kNE];
 #pragma unroll
-                for (int q = 0; q < 8; q++) xn[q] = xc[q];
-                if (kk + 8 < kKC) fetch(kk + 8, wn, xn);
-                const uint32_t ww[4] = {wc.x, wc.y, wc.z, wc.w};
+            for (int j = 0; j < kNE; j++) wq[j] = *reinterpret_cast<const uint4*>(wrow + j * 32 * kNWStride + kk * 2);
 #pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    const float2 w2 = bf16x2_to_f32(ww[q]);
-                    const float4 xa = xc[2 * q], xb = xc[2 * q + 1];
-                    acc[0] = __fmaf_rn(xa.x, w2.x, acc[0]);
-                    acc[1] = __fmaf_rn(xa.y, w2.x, acc[1]);
-                    acc[2] = __fmaf_rn(xa.z, w2.x, acc[2]);
-                    acc[3] = __fmaf_rn(xa.w, w2.x, acc[3]);
-                    acc[0] = __fmaf_rn(xb.x, w2.y, acc[0]);
-                    acc[1] = __fmaf_rn(xb.y, w2.y, acc[1]);
-                    acc[2] = __fmaf_rn(xb.z, w2.y, acc[2]);
-                    acc[3] = __fmaf_rn(xb.w, w2.y, acc[3]);
+            for (int q = 0; q < 8; q++) {
+                const float4 x4 = *reinterpret_cast<const float4*>(xs + (kk + q) * kNTok);
+                const float xv[kNT] = {x4.x, x4.y, x4.z, x4.w};
+#pragma unroll
+                for (int j = 0; j < kNE; j++) {
+                    const uint32_t pair = (q < 2) ? wq[j].x : (q < 4) ? wq[j].y : (q < 6) ? wq[j].z : wq[j].w;
+                    const float wv = __uint_as_float((q & 1) ? (pair & 0xffff0000u) : (pair << 16));
+#pragma unroll
+                    for (int i = 0; i < kNT; i++) acc[j][i] = __fmaf_rn(xv[i], wv, acc[j][i]);
                 }
-                wc = wn;
-#pragma unroll
-                for (int q = 0; q < 8; q++) xc[q] = xn[q];
             }
         }
         if (c + 1 < nchunks) store_x(b ^ 1);
     }
-    const int e = e0 + lane;
-    if (active && e < experts) {
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const int t = t0 + warp * 4 + i;
-            if (t < tokens) logits[(size_t)t * experts + e] = acc[i];
+    for (int j = 0; j < kNE; j++) {
+        const int e = e0 + lane + 32 * j;
+        if (e < experts) {
+#pragma unroll
+            for (int i = 0; i < kNT; i++) {
+                const int t = t0 + warp * kNT + i;
+                if (t < tokens) logits[(size_t)t * experts + e] = acc[j][i];
+            }
         }
     }
 }
@@ -299,91 +290,77 @@ router_topk_kernel(const float* __restrict__ logits, int tokens, int experts, in
 // tokens/4 x 8 CTAs and the chain of 2048 dependent FMAs is the only long latency), stores them into the
 // first CTA's shared memory (distributed shared memory), and after the cluster barrier the first CTA's four
 // warps run the top-k of the four tokens.  Same arithmetic, same order as the two separate kernels.
-constexpr int kFusedTok = 4, kFusedK = 256;
+// The gate rows come cold from HBM: with one chunk of 256 k ahead every chunk waited for its load (8 tokens 12.7 us, 64
+// tokens 17.2), so the ring keeps kFusedStages chunks of 128 k in flight (11.6 and 15.3) and the chain, 32 cycles
+// per eight k, is the larger part of what is left.
+constexpr int kFusedTok = 4, kFusedK = 128, kFusedStages = 6;
 constexpr int kFusedWStride = kFusedK * 2 + 16;
+constexpr int kFusedStageBytes = 32 * kFusedWStride + kFusedTok * kFusedK * 2;
+constexpr int kFusedSmem = kFusedStages * kFusedStageBytes + kFusedTok * 256 * 4;
 
 __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(128)
 router_fused_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gate_w, int tokens,
                     int hidden, int top_k, int32_t* __restrict__ ids, float* __restrict__ weights) {
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
-    __shared__ __align__(16) uint8_t wbuf[2][32 * kFusedWStride];
-    __shared__ __align__(16) float xbuf[2][kFusedTok][kFusedK];
-    __shared__ float slog[kFusedTok][256];       // used in the cluster's first CTA
+    extern __shared__ __align__(16) uint8_t rsm[];                                        // [stages][gate rows | token rows]
+    float* const slog = reinterpret_cast<float*>(rsm + kFusedStages * kFusedStageBytes);   // [tok][256], the cluster's first CTA
     pdl_launch_dependents();
     const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
     const int rank = (int)cluster.block_rank();   // = blockIdx.x: experts 32 * rank ..
     const int e0 = rank * 32, t0 = blockIdx.y * kFusedTok;
     const int nchunks = hidden / kFusedK;
-    const uint32_t wbase = (uint32_t)__cvta_generic_to_shared(&wbuf[0][0]);
+    const uint32_t base = (uint32_t)__cvta_generic_to_shared(rsm);
 
-    auto issue_w = [&](int c, int b) {
-        for (int i = tid; i < 32 * (kFusedK / 8); i += 128) {
-            const int row = i / (kFusedK / 8), piece = i % (kFusedK / 8);
-            cp_async16(wbase + b * 32 * kFusedWStride + row * kFusedWStride + piece * 16,
-                       gate_w + (size_t)(e0 + row) * hidden + c * kFusedK + piece * 8);
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-    // activations of the chunk: thread -> token tid / 32, 8 k at lane * 8
-    uint4 xr;
-    auto load_x = [&](int c) {
-        const int t = t0 + warp;
-        xr = make_uint4(0, 0, 0, 0);
-        if (t < tokens) xr = *reinterpret_cast<const uint4*>(x + (size_t)t * hidden + c * kFusedK + lane * 8);
-    };
-    auto store_x = [&](int b) {
-        const uint32_t w[4] = {xr.x, xr.y, xr.z, xr.w};
-        float* dst = &xbuf[b][warp][lane * 8];
+    auto issue = [&](int c) {
+        if (c < nchunks) {
+            const uint32_t st = base + (c % kFusedStages) * kFusedStageBytes;
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
-            const float2 v = bf16x2_to_f32(w[q]);
-            dst[2 * q] = v.x;
-            dst[2 * q + 1] = v.y;
+            for (int i = 0; i < 32 * (kFusedK / 8) / 128; i++) {
+                const int row = (tid + i * 128) / (kFusedK / 8), piece = (tid + i * 128) % (kFusedK / 8);
+                cp_async16(st + row * kFusedWStride + piece * 16, gate_w + (size_t)(e0 + row) * hidden + c * kFusedK + piece * 8);
+            }
+            if (tid < kFusedTok * (kFusedK / 8)) {
+                const int row = tid / (kFusedK / 8), piece = tid % (kFusedK / 8);
+                // a token past the end repeats the last one; its result is not stored
+                cp_async16(st + 32 * kFusedWStride + row * kFusedK * 2 + piece * 16,
+                           x + (size_t)min(t0 + row, tokens - 1) * hidden + c * kFusedK + piece * 8);
+            }
         }
+        asm volatile("cp.async.commit_group;" ::: "memory");      // one group per chunk, empty past the end
     };
-    issue_w(0, 0);
-    load_x(0);
-    store_x(0);
+#pragma unroll
+    for (int c = 0; c < kFusedStages - 1; c++) issue(c);
     float acc = 0.f;
     for (int c = 0; c < nchunks; c++) {
-        const int b = c & 1;
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        __syncthreads();
-        if (c + 1 < nchunks) {
-            issue_w(c + 1, b ^ 1);
-            load_x(c + 1);
-        }
-        const uint32_t wrow = wbase + b * 32 * kFusedWStride + lane * kFusedWStride;
-        const float* xs = &xbuf[b][warp][0];
-#pragma unroll 4
+        asm volatile("cp.async.wait_group %0;" ::"n"(kFusedStages - 2) : "memory");
+        __syncthreads();                                          // chunk c is there for all, chunk c - 1 is done with
+        issue(c + kFusedStages - 1);
+        const uint8_t* const st = rsm + (c % kFusedStages) * kFusedStageBytes;
+        const uint8_t* const wrow = st + lane * kFusedWStride;
+        const uint8_t* const xrow = st + 32 * kFusedWStride + warp * kFusedK * 2;
+#pragma unroll
         for (int kk = 0; kk < kFusedK; kk += 8) {
-            uint4 wv;
-            asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(wv.x), "=r"(wv.y), "=r"(wv.z), "=r"(wv.w) : "r"(wrow + kk * 2));
-            const float4 xa = *reinterpret_cast<const float4*>(xs + kk), xb = *reinterpret_cast<const float4*>(xs + kk + 4);
-            const float2 w01 = bf16x2_to_f32(wv.x), w23 = bf16x2_to_f32(wv.y), w45 = bf16x2_to_f32(wv.z), w67 = bf16x2_to_f32(wv.w);
-            acc = __fmaf_rn(xa.x, w01.x, acc);
-            acc = __fmaf_rn(xa.y, w01.y, acc);
-            acc = __fmaf_rn(xa.z, w23.x, acc);
-            acc = __fmaf_rn(xa.w, w23.y, acc);
-            acc = __fmaf_rn(xb.x, w45.x, acc);
-            acc = __fmaf_rn(xb.y, w45.y, acc);
-            acc = __fmaf_rn(xb.z, w67.x, acc);
-            acc = __fmaf_rn(xb.w, w67.y, acc);
+            const uint4 wv = *reinterpret_cast<const uint4*>(wrow + kk * 2);
+            const uint4 xv = *reinterpret_cast<const uint4*>(xrow + kk * 2);
+            const uint32_t ww[4] = {wv.x, wv.y, wv.z, wv.w}, xx[4] = {xv.x, xv.y, xv.z, xv.w};
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const float2 w2 = bf16x2_to_f32(ww[q]), x2 = bf16x2_to_f32(xx[q]);
+                acc = __fmaf_rn(x2.x, w2.x, acc);
+                acc = __fmaf_rn(x2.y, w2.y, acc);
+            }
         }
-        if (c + 1 < nchunks) store_x(b ^ 1);
     }
     // hand the logit to the cluster's first CTA
-    float* remote = cluster.map_shared_rank(&slog[0][0], 0);
+    float* remote = cluster.map_shared_rank(slog, 0);
     remote[warp * 256 + e0 + lane] = acc;
     cluster.sync();
     if (rank == 0) {
         const int t = t0 + warp;
-        if (t < tokens) warp_topk_row<8>(&slog[warp][0], 256, top_k, lane, ids + (size_t)t * top_k, weights + (size_t)t * top_k);
+        if (t < tokens) warp_topk_row<8>(slog + warp * 256, 256, top_k, lane, ids + (size_t)t * top_k, weights + (size_t)t * top_k);
     }
 }
-
-
 
 // ---- wide variant for large batches --------------------------------------------------------
 // CTA = 4 warps, tile = 64 experts x 32 tokens; a lane owns experts lane and lane + 32, a warp 8 tokens:
@@ -597,10 +574,22 @@ router_logits_big_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat1
     }
 }
 
+template <int NE>
+void launch_narrow(const __nv_bfloat16* x, const __nv_bfloat16* gate_w, int tokens, int experts, int hidden, float* logits,
+                   const Ctx& c) {
+    constexpr size_t smem = 2 * 32 * NE * kNWStride + 2 * kNK * kNTok * sizeof(float);
+    const dim3 grid((experts + 32 * NE - 1) / (32 * NE), (tokens + kNTok - 1) / kNTok);
+    static PerDeviceOnce once;
+    allow_dyn_smem(once, router_logits_narrow_kernel<NE>, smem);
+    c.begin(K_ROUTER_LOGITS);
+    router_logits_narrow_kernel<NE><<<grid, 128, smem, c.s>>>(x, gate_w, tokens, experts, hidden, logits);
+    c.end();
+}
+
 }  // namespace
 
 int launch_router_logits(const __nv_bfloat16* x, const __nv_bfloat16* gate_w, int tokens, int experts,
-                         int hidden, float* logits, const Ctx& c) {
+                         int hidden, float* logits, int sm_count, const Ctx& c) {
     if (hidden % kGK == 0 && tokens >= 4096 && experts >= kGE) {
         dim3 grid((experts + kGE - 1) / kGE, (tokens + kGT - 1) / kGT);
         const size_t smem = 2 * kGE * kGWStride + 2 * kGK * kGT * sizeof(float);
@@ -611,8 +600,13 @@ int launch_router_logits(const __nv_bfloat16* x, const __nv_bfloat16* gate_w, in
         c.end();
         return 1;
     }
-    if (hidden % kBK == 0 && tokens >= 768) {      // below that the 32 x 16 tiles fill the device better
-        dim3 grid((experts + kBE - 1) / kBE, (tokens + kBT - 1) / kBT);
+    // The wide kernel from 768 tokens (below, its 64 x 32 tiles leave SMs idle: 512 tokens 31.5 us against 49), except
+    // where its tiles just miss one per SM and most SMs would wait for a second round: 1500 tokens (188 tiles) take
+    // 69.5 us with the narrow kernel, 83 with the wide one; 2048 (256 tiles) 92 against 83.5.
+    const dim3 grid((experts + kBE - 1) / kBE, (tokens + kBT - 1) / kBT);
+    const int tiles = (int)(grid.x * grid.y);
+    const bool short_round = tiles > sm_count && tiles * 10 < sm_count * 14;
+    if (hidden % kBK == 0 && tokens >= 768 && !(short_round && hidden % 256 == 0)) {
         const size_t smem = 2 * kBE * kBWStride + 2 * kBK * kBT * sizeof(float);
         static PerDeviceOnce once;
         allow_dyn_smem(once, router_logits_wide_kernel, smem);
@@ -621,14 +615,11 @@ int launch_router_logits(const __nv_bfloat16* x, const __nv_bfloat16* gate_w, in
         c.end();
         return 1;
     }
-    if (hidden % kKC == 0) {
-        dim3 grid((experts + kTileE - 1) / kTileE, (tokens + kTileT - 1) / kTileT);
-        const size_t smem = 2 * kTileE * kWStride + 2 * kKC * kTileT * sizeof(float);
-        static PerDeviceOnce once;
-        allow_dyn_smem(once, router_logits_tiled_kernel, smem);
-        c.begin(K_ROUTER_LOGITS);
-        router_logits_tiled_kernel<<<grid, 128, smem, c.s>>>(x, gate_w, tokens, experts, hidden, logits);
-        c.end();
+    if (hidden % 256 == 0) {
+        if ((experts + 31) / 32 * ((tokens + kNTok - 1) / kNTok) <= sm_count)
+            launch_narrow<1>(x, gate_w, tokens, experts, hidden, logits, c);
+        else
+            launch_narrow<2>(x, gate_w, tokens, experts, hidden, logits, c);
         return 1;
     }
     dim3 block(kExpertsPerCta, kTokGroups);
@@ -653,17 +644,18 @@ int launch_router_logits(const __nv_bfloat16* x, const __nv_bfloat16* gate_w, in
 }
 
 bool router_fused_supported(int tokens, int experts, int hidden, int top_k) {
-    // measured per whole block (Zipf routing): 128 tokens 105 us fused against 115 us with the tiled kernel + top-k,
-    // 256 tokens 157 against 147, 512 tokens 194 against 189: the cluster kernel re-reads the gate weight once per
-    // four tokens and walks one chain per thread, which stops paying at about 200 tokens
-    return experts == 256 && hidden % kFusedK == 0 && tokens < 256 && top_k <= 32;
+    // router alone: 128 tokens 15.6 us, 173 tokens 21.4, 200 tokens 27.0 here; 25.5 from 1 to 288 tokens with the narrow
+    // kernel and the separate top-k.  The cluster kernel re-reads the gate weight once per four tokens.
+    return experts == 256 && hidden % 256 == 0 && tokens < 192 && top_k <= 32;
 }
 
 int launch_router_fused(const __nv_bfloat16* x, const __nv_bfloat16* gate_w, int tokens, int hidden, int top_k,
                         int32_t* ids, float* weights, const Ctx& c) {
     dim3 grid(8, (tokens + kFusedTok - 1) / kFusedTok);
+    static PerDeviceOnce once;
+    allow_dyn_smem(once, router_fused_kernel, kFusedSmem);
     c.begin(K_ROUTER_LOGITS);
-    router_fused_kernel<<<grid, 128, 0, c.s>>>(x, gate_w, tokens, hidden, top_k, ids, weights);
+    router_fused_kernel<<<grid, 128, kFusedSmem, c.s>>>(x, gate_w, tokens, hidden, top_k, ids, weights);
     c.end();
     return 1;
 }

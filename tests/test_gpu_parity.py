@@ -117,6 +117,37 @@ def test_router_ids_bit_exact_full(full, tokens):
     assert np.abs(w.cpu().numpy() - want_w).max() <= 1e-6
 
 
+def test_router_ids_bit_exact_at_the_borders_of_its_kernels():
+    """Token counts either side of every rule: the cluster kernel, tiles of 16 tokens, tiles of 32 where they fill the
+    device, and the range where those would leave most SMs waiting for a second round.  A row's ids and weights depend
+    on that row alone, so one run of the CPU path serves all counts; equal bit for bit."""
+    lay = pkg.synth.make_layer(32, hidden=2048, inter=512, experts=256, top_k=8, shared_inter=512)
+    moe = pkg.B200MoE(0, pkg.ExpertShapes(2048, 512), 1, experts=256, layers=1, top_k=8, shared_inter=0, max_tokens=2100)
+    xb = pkg.synth.make_x(4243, 2100, lay.hidden)
+    want_ids, want_w = o.router(oracle_layer(lay), pkg.synth.bf16_bits_to_f32(xb))
+    x, gate = bf16_dev(xb), bf16_dev(lay.gate_w)
+    for tokens in (3, 4, 5, 130, 191, 192, 193, 287, 288, 289, 513, 767, 768, 1184, 1185, 1500, 1656, 1657, 1697, 2100):
+        ids, w = moe.router(x[:tokens], gate)
+        assert np.array_equal(ids.cpu().numpy(), want_ids[:tokens]), tokens
+        assert np.array_equal(w.cpu().numpy(), want_w[:tokens]), tokens
+    moe.close()
+
+
+@pytest.mark.parametrize("hidden,experts,top_k", [(256, 256, 8), (768, 256, 4), (256, 100, 8), (512, 300, 6)])
+def test_router_ids_bit_exact_other_widths(hidden, experts, top_k):
+    """Two to six chunks of k (fewer than the cluster kernel keeps in flight), a last tile of experts that is not full."""
+    lay = pkg.synth.make_layer(33, hidden=hidden, inter=16, experts=experts, top_k=top_k, shared_inter=16)
+    moe = pkg.B200MoE(0, pkg.ExpertShapes(hidden, 16), 1, experts=experts, layers=1, top_k=top_k, shared_inter=0, max_tokens=333)
+    xb = pkg.synth.make_x(4244, 333, hidden)
+    want_ids, want_w = o.router(oracle_layer(lay), pkg.synth.bf16_bits_to_f32(xb))
+    x, gate = bf16_dev(xb), bf16_dev(lay.gate_w)
+    for tokens in (1, 17, 333):
+        ids, w = moe.router(x[:tokens], gate)
+        assert np.array_equal(ids.cpu().numpy(), want_ids[:tokens]), tokens
+        assert np.array_equal(w.cpu().numpy(), want_w[:tokens]), tokens
+    moe.close()
+
+
 def test_router_ids_bit_exact_at_4200_tokens():
     """Batches of 4096 tokens and more take a kernel of their own (32 chains per thread); 4200 tokens leave a
     ragged last tile of eight.  Ids and weights equal the CPU path's bit for bit."""
