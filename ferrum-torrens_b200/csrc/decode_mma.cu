@@ -903,10 +903,9 @@ __global__ void scale_repack_kernel(const uint8_t* __restrict__ scale /* the slo
     *reinterpret_cast<uint4*>(dst + ((size_t)(tile * groups + q) * 32 + lane) * 16) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
 }
 
-// latency-bound steps (a handful of tokens) chain their kernels with programmatic dependent launch: measured
-// 49 -> 43 us per block at one token; at 64 tokens the early-resident CTAs only get in the way of the shared
-// expert that runs beside them, so larger steps launch the ordinary way
-constexpr int kPdlMaxRoutes = 128;
+// Plan, gate_up and down are chained with programmatic dependent launch: each sets up under the tail of the one before
+// (a block at one token 49 -> 43 us, 37 tokens 84.5 -> 80.7, 173 tokens 118.7 -> 115.9).  From 64 tokens on it used to
+// lose, because the early-resident CTAs kept the shared expert off the SMs; that is done before they come now.
 constexpr int kDefaultVariant = 14;   // register-streaming kernels, fragment-ordered scales, 256-byte L2 fill
 
 template <bool GATE_UP, int K_, int NT, int OCC, int VAR>
@@ -1058,10 +1057,7 @@ int launch_decode_mma(const BankView& b, const void* x, int x_dtype, const Decod
         static PerDeviceOnce once;
         allow_dyn_smem(once, decode_plan_kernel, 200 * 1024);
         c.begin(K_DECODE_PLAN);
-        if (routes <= kPdlMaxRoutes)
-            launch_pdl(decode_plan_kernel, dim3(1), dim3(kPlanThreads), psmem, c.s, pa);
-        else
-            decode_plan_kernel<<<1, kPlanThreads, psmem, c.s>>>(pa);
+        launch_pdl(decode_plan_kernel, dim3(1), dim3(kPlanThreads), psmem, c.s, pa);
         c.end();
         launches += 1;
     } else {
@@ -1099,7 +1095,7 @@ int launch_decode_mma(const BankView& b, const void* x, int x_dtype, const Decod
     a.act = x; a.act_dtype = x_dtype; a.ic2 = sc.ic2p; a.N = 2 * b.inter;
     c.begin(K_EXPERT_GATE_UP);
     if (small)
-        launch_expert<true, 2048, 1, 1>(a, sm_count, c.s, routes <= kPdlMaxRoutes);
+        launch_expert<true, 2048, 1, 1>(a, sm_count, c.s, true);
     else
         launch_expert<true, 2048, 2, 1>(a, sm_count, c.s, false);
     c.end();
@@ -1108,7 +1104,7 @@ int launch_decode_mma(const BankView& b, const void* x, int x_dtype, const Decod
     a.act = sc.ic2p; a.act_dtype = 1; a.yroute = sc.yroute; a.route_weight = route_weight; a.N = b.hidden;
     c.begin(K_EXPERT_DOWN);
     if (small)
-        launch_expert<false, 512, 1, 1>(a, sm_count, c.s, routes <= kPdlMaxRoutes);
+        launch_expert<false, 512, 1, 1>(a, sm_count, c.s, true);
     else
         launch_expert<false, 512, 2, 1>(a, sm_count, c.s, false);
     c.end();
