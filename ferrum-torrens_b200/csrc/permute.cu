@@ -153,6 +153,8 @@ __global__ void __launch_bounds__(kThreads)
 csr_count_kernel(const int32_t* route_bin, int routes, int bins, int chunk, int32_t* __restrict__ cta_hist,
                  int32_t* bad_flag, SlotRewrite w) {
     extern __shared__ int sm[];
+    pdl_launch_dependents();
+    pdl_wait();
     if (w.expert_ids) {
         const int begin = blockIdx.x * chunk, end = min(begin + chunk, routes);
         for (int r = begin + threadIdx.x; r < end; r += kThreads) rewrite_route(w, r);
@@ -174,6 +176,8 @@ __global__ void __launch_bounds__(kMaxBins)
 csr_scan_kernel(int32_t* __restrict__ cta_hist, int nctas, int bins, int32_t* __restrict__ seg, CsrGroups g) {
     __shared__ int wsum[32];
     const int b = threadIdx.x;
+    pdl_launch_dependents();
+    pdl_wait();
     int total = 0;
     if (b < bins)
         for (int c = 0; c < nctas; c++) total += cta_hist[(size_t)c * bins + b];
@@ -248,6 +252,8 @@ csr_scatter_kernel(const int32_t* __restrict__ route_bin, int routes, int bins, 
                    const int32_t* __restrict__ cta_base, int32_t* __restrict__ route_idx, int32_t* scratch_flag,
                    int32_t* __restrict__ pos_of_route) {
     extern __shared__ int sm[];
+    pdl_launch_dependents();
+    pdl_wait();
     count_chunk(route_bin, routes, bins, blockIdx.x * chunk, chunk / kWarps, sm, scratch_flag);
     for (int b = threadIdx.x; b < bins; b += kThreads) {
         int run = cta_base[(size_t)blockIdx.x * bins + b];
@@ -314,12 +320,13 @@ int launch_csr_build(const int32_t* route_bin, int routes, int bins, int32_t* se
     int nctas = (routes + chunk - 1) / chunk;
     size_t smem = (size_t)kWarps * bins * sizeof(int);
     c.begin(K_CSR);
-    csr_count_kernel<<<nctas, kThreads, smem, c.s>>>(route_bin, routes, bins, chunk, scratch, bad_flag,
-                                                     rewrite ? *rewrite : SlotRewrite{});
+    // programmatic dependent launch: three kernels of 3 us each, with 3 us between them when launched the ordinary way
+    launch_pdl(csr_count_kernel, dim3(nctas), dim3(kThreads), smem, c.s, route_bin, routes, bins, chunk, scratch, bad_flag,
+               rewrite ? *rewrite : SlotRewrite{});
     int scan_threads = ((bins + 31) / 32) * 32;
-    csr_scan_kernel<<<1, scan_threads, 0, c.s>>>(scratch, nctas, bins, seg, groups ? *groups : CsrGroups{});
-    csr_scatter_kernel<<<nctas, kThreads, smem, c.s>>>(route_bin, routes, bins, chunk, scratch, route_idx, bad_flag,
-                                                       groups ? groups->pos_of_route : nullptr);
+    launch_pdl(csr_scan_kernel, dim3(1), dim3(scan_threads), 0, c.s, scratch, nctas, bins, seg, groups ? *groups : CsrGroups{});
+    launch_pdl(csr_scatter_kernel, dim3(nctas), dim3(kThreads), smem, c.s, route_bin, routes, bins, chunk, scratch, route_idx,
+               bad_flag, groups ? groups->pos_of_route : nullptr);
     c.end();
     return 3;
 }

@@ -37,6 +37,8 @@
 // Every mbarrier wait is bounded; a wait that gives up raises the error flag and the CTA drains.
 #include <cuda.h>
 
+#include <algorithm>
+
 #include "kernels.cuh"
 #include "umma.cuh"
 
@@ -76,14 +78,20 @@ __device__ __forceinline__ uint32_t hmul2_f16(uint32_t a, uint32_t b) {
 }
 
 // ---- gather: sorted activations as scaled f16 ------------------------------------------------
-// one warp per sorted position (no block-wide synchronisation); K == 2048: a lane holds 8 chunks of 8 k
+// Part `p` of token t (one warp each, no block-wide synchronisation) reads the token's row once, scales it, and writes
+// it at the sorted positions of the token's routes p, p + parts, ..; K == 2048: a lane holds 8 chunks of 8 k.  Bound by
+// the writes (top_k rows of 4 KB per token): one warp per sorted row read and converted every row top_k times (8192
+// tokens: 60 us).  Small batches cut a token's routes into parts to have warps for every SM.
 __global__ void __launch_bounds__(256)
-prefill_gather_kernel(const void* __restrict__ x, int x_dtype, const int32_t* __restrict__ route_idx,
-                      const int32_t* __restrict__ n_sorted, int top_k, int K, __half* __restrict__ xg,
+prefill_gather_kernel(const void* __restrict__ x, int x_dtype, const int32_t* __restrict__ bin_of_route, int nbins,
+                      const int32_t* __restrict__ pos_of_route, int tokens, int top_k, int parts, int K, __half* __restrict__ xg,
                       float* __restrict__ row_scale) {
-    const int i = blockIdx.x * 8 + threadIdx.x / 32, lane = threadIdx.x % 32;
-    if (i >= *n_sorted) return;   // routes of unknown experts are in no bucket
-    const size_t src = (size_t)(route_idx[i] / top_k) * K;
+    const int w = blockIdx.x * 8 + threadIdx.x / 32, lane = threadIdx.x % 32;
+    const int t = w / parts, part = w % parts;
+    pdl_launch_dependents();
+    pdl_wait();
+    if (t >= tokens) return;
+    const size_t src = (size_t)t * K;
     constexpr int kChunksPerLane = 8;   // 2048 / (32 lanes * 8 k)
     float v[kChunksPerLane][8];
     float m = 0.f;
@@ -124,16 +132,22 @@ prefill_gather_kernel(const void* __restrict__ x, int x_dtype, const int32_t* __
         inv = __uint_as_float((uint32_t)(127 + 14 - (e - 127)) << 23);
         sc = __uint_as_float((uint32_t)(127 - 14 + (e - 127)) << 23);
     }
+    __half2 h[kChunksPerLane][4];
 #pragma unroll
-    for (int c = 0; c < kChunksPerLane; c++) {
-        __half2 h[4];
+    for (int c = 0; c < kChunksPerLane; c++)
 #pragma unroll
-        for (int q = 0; q < 4; q++) h[q] = __floats2half2_rn(v[c][2 * q] * inv, v[c][2 * q + 1] * inv);
-        *reinterpret_cast<uint4*>(xg + (size_t)i * K + (c * 32 + lane) * 8) =
-            make_uint4(*reinterpret_cast<uint32_t*>(&h[0]), *reinterpret_cast<uint32_t*>(&h[1]),
-                       *reinterpret_cast<uint32_t*>(&h[2]), *reinterpret_cast<uint32_t*>(&h[3]));
+        for (int q = 0; q < 4; q++) h[c][q] = __floats2half2_rn(v[c][2 * q] * inv, v[c][2 * q + 1] * inv);
+    for (int j = part; j < top_k; j += parts) {
+        const int r = t * top_k + j, bin = bin_of_route[r];
+        if (bin < 0 || bin >= nbins) continue;     // a route of an unknown expert is in no bucket
+        const int i = pos_of_route[r];
+#pragma unroll
+        for (int c = 0; c < kChunksPerLane; c++)
+            *reinterpret_cast<uint4*>(xg + (size_t)i * K + (c * 32 + lane) * 8) =
+                make_uint4(*reinterpret_cast<uint32_t*>(&h[c][0]), *reinterpret_cast<uint32_t*>(&h[c][1]),
+                           *reinterpret_cast<uint32_t*>(&h[c][2]), *reinterpret_cast<uint32_t*>(&h[c][3]));
+        if (lane == 0) row_scale[i] = sc;
     }
-    if (lane == 0) row_scale[i] = sc;
 }
 
 // ic1 (f32, sorted rows: gate | up) -> ic2 = silu(gate) * up as f16 with a per-row power-of-two scale.
@@ -142,6 +156,8 @@ __global__ void __launch_bounds__(256)
 prefill_rescale_kernel(const float* __restrict__ ic1, const int32_t* __restrict__ n_sorted, int K,
                        __half* __restrict__ ic2h, float* __restrict__ row_scale) {
     const int row = blockIdx.x * 8 + threadIdx.x / 32, lane = threadIdx.x % 32;
+    pdl_launch_dependents();
+    pdl_wait();
     if (row >= *n_sorted) return;
     float v[16];
     float m = 0.f;
@@ -207,7 +223,27 @@ constexpr int kRawScaleBytes = kTileM * 16;    // 128 rows x 16 scale bytes (256
 constexpr int kRawStageBytes = kRawPackedBytes + kRawScaleBytes;
 constexpr int kWBufs = kMaxDeqSets;            // dequantised weight chunks in tensor memory, 64 columns each
 constexpr int kWCols = 64;
-constexpr int kAccCol0 = kWBufs * kWCols;      // accumulators: a ring of two tiles of 128 f32 columns behind them
+constexpr int kAccCol0 = kWBufs * kWCols;      // accumulators behind them: per row tile two slots of 64 f32 columns
+constexpr int kAccSlot = 64;
+
+// Which accumulator slots a unit takes.  A pass of at most 64 rows takes one slot, in turn, so that its epilogue runs
+// under the next unit's MMAs; a longer one takes both (128 columns).  Every role walks the same units and keeps this
+// count for itself; a slot's barriers complete once per unit that takes it.
+struct AccCursor {
+    uint32_t used[2] = {0, 0};   // units that have taken the slot so far
+    int next = 0;
+    int first, last;             // slots of the current unit
+    __device__ __forceinline__ void take(int rows) {
+        first = rows > kAccSlot ? 0 : next;
+        last = rows > kAccSlot ? 1 : next;
+        if (rows <= kAccSlot) next ^= 1;
+    }
+    __device__ __forceinline__ uint32_t parity(int slot) const { return (slot ? used[1] : used[0]) & 1; }
+    __device__ __forceinline__ void done() {
+        if (first == 0) used[0]++;
+        if (last == 1) used[1]++;
+    }
+};
 
 // activation tile maps by box height: 32, 64, 96 or 128 token rows, so that a small group does not
 // pull 128 rows through L2
@@ -233,6 +269,7 @@ umma_grouped_gemm_kernel(const __grid_constant__ XMaps xmaps, const __grid_const
     constexpr int kRS = RET ? kRawStages - 1 : kRawStages;   // the owner's variant gives a raw stage to its epilogue staging
     constexpr int kWarpEpi2 = kWarpDeq0 + 4 * kDeqSets;     // down: warps 16..19 row tile 0, 20..23 row tile 1
     extern __shared__ uint8_t smem_raw[];
+    pdl_launch_dependents();
     // 1024-byte alignment for the swizzled tiles
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     uint8_t* const x_tiles = smem;                                         // [kXStages][16 KiB]: 128 tokens x 64 k
@@ -250,7 +287,8 @@ umma_grouped_gemm_kernel(const __grid_constant__ XMaps xmaps, const __grid_const
     auto RAW_EMPTY = [&](int s) { return bar0 + 8u * (22 + s); };
     auto W_READY = [&](int s) { return bar0 + 8u * (28 + s); };          // kWBufs <= 4
     auto W_FREE = [&](int s) { return bar0 + 8u * (32 + s); };
-    const uint32_t ACC_FULL = bar0 + 8u * 36, ACC_EMPTY = bar0 + 8u * 37;
+    auto ACC_FULL = [&](int s) { return bar0 + 8u * (36 + s); };         // per accumulator slot
+    auto ACC_EMPTY = [&](int s) { return bar0 + 8u * (38 + s); };
 
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     if (threadIdx.x == 0) {
@@ -266,8 +304,10 @@ umma_grouped_gemm_kernel(const __grid_constant__ XMaps xmaps, const __grid_const
             mbar_init(W_READY(s), 128);
             mbar_init(W_FREE(s), 1);
         }
-        mbar_init(ACC_FULL, 2);
-        mbar_init(ACC_EMPTY, kEpiSets * 128);
+        for (int s = 0; s < 2; s++) {
+            mbar_init(ACC_FULL(s), 2);
+            mbar_init(ACC_EMPTY(s), kEpiSets * 128);
+        }
         *s_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -286,6 +326,7 @@ umma_grouped_gemm_kernel(const __grid_constant__ XMaps xmaps, const __grid_const
     static_assert(kItems % kDeqSets == 0, "every dequantiser set sees the same pieces of every unit");
     static_assert(kWBufs % kDeqSets == 0, "a weight buffer belongs to one dequantiser set");
     const int n_pairs = a.N / (2 * kTileM);
+    pdl_wait();     // barriers and tensor memory are set up under the tail of the kernel before
     const int n_units = *a.n_groups * n_pairs;
 
     if (warp == kWarpActTma) {
@@ -343,19 +384,22 @@ umma_grouped_gemm_kernel(const __grid_constant__ XMaps xmaps, const __grid_const
         // token tile takes.
         {
             const int r = (warp == kWarpMma) ? 0 : 1;
-            const uint32_t d_tmem = tmem_base + kAccCol0 + r * kTileTok;
-            uint32_t it = 0, item = r, unit_i = 0;
+            uint32_t it = 0, item = r;
+            AccCursor acc;
             // Looking at a barrier costs a shared-memory round trip even when its phase completed long ago, and
             // this warp's chain (look, issue, look, issue ..) is what the tensor pipe waits for at small token
             // tiles.  So the barriers of the NEXT step are looked at (without suspending) just before this
             // step's MMAs are issued, and the blocking wait is taken only when that look came back empty.
             bool x_seen = false, w_seen = false;
-            for (int u = blockIdx.x; u < n_units && !*s_abort; u += gridDim.x, unit_i++) {
+            for (int u = blockIdx.x; u < n_units && !*s_abort; u += gridDim.x, acc.done()) {
                 const int4 grp = a.groups[u / n_pairs];
+                acc.take(grp.z);
+                const uint32_t d_tmem = tmem_base + kAccCol0 + r * kTileTok + acc.first * kAccSlot;
                 const int n_pad = max(16, (grp.z + 15) & ~15);
                 const uint32_t idesc = kIdescBase | ((uint32_t)(n_pad >> 3) << 17);
                 // the accumulators must have been read back
-                bool ok = mbar_wait_warp(ACC_EMPTY, (unit_i & 1) ^ 1, s_abort, a.err);
+                bool ok = mbar_wait_warp(ACC_EMPTY(acc.first), acc.parity(acc.first) ^ 1, s_abort, a.err);
+                if (ok && acc.last != acc.first) ok = mbar_wait_warp(ACC_EMPTY(acc.last), acc.parity(acc.last) ^ 1, s_abort, a.err);
                 for (int ks = 0; ks < 2 * kChunks && ok; ks++, it++) {
                     const int h = ks & 1;                        // half of the 128-k weight piece
                     const int wb = item % kWBufs;
@@ -386,7 +430,10 @@ umma_grouped_gemm_kernel(const __grid_constant__ XMaps xmaps, const __grid_const
                     if (h == 1) item += 2;
                 }
                 if (!ok) break;
-                if (elect_one()) umma_commit(ACC_FULL);
+                if (elect_one()) {
+                    umma_commit(ACC_FULL(acc.first));
+                    if (acc.last != acc.first) umma_commit(ACC_FULL(acc.last));
+                }
                 __syncwarp();
             }
         }
@@ -462,10 +509,11 @@ umma_grouped_gemm_kernel(const __grid_constant__ XMaps xmaps, const __grid_const
             const int r = (warp < kWarpDeq0) ? 0 : (warp >= kWarpEpi1) ? 1 : ((warp - kWarpEpi2) >> 2);
             const int half = (warp >= kWarpDeq0 && warp < kWarpEpi1) ? 1 : 0;
             constexpr int kStride = 16 * (kEpiSets / 2);
-            uint32_t unit_i = 0;
-            for (int u = blockIdx.x; u < n_units && !*s_abort; u += gridDim.x, unit_i++) {
+            AccCursor acc;
+            for (int u = blockIdx.x; u < n_units && !*s_abort; u += gridDim.x, acc.done()) {
                 const int4 grp = a.groups[u / n_pairs];
                 const int cnt = grp.z, pos0 = grp.y;
+                acc.take(cnt);
                 const int wrow = (u % n_pairs) * 2 * kTileM + r * kTileM + quarter * 32 + lane;
                 const float gl = f16_global_to_f32(a.global[(size_t)grp.x * a.N + wrow]);
                 float fac[4];
@@ -479,10 +527,11 @@ umma_grouped_gemm_kernel(const __grid_constant__ XMaps xmaps, const __grid_const
                     }
                     fac[q] = f;
                 }
-                if (!mbar_wait(ACC_FULL, unit_i & 1, s_abort, a.err)) break;
+                if (!mbar_wait(ACC_FULL(acc.first), acc.parity(acc.first), s_abort, a.err)) break;
+                if (acc.last != acc.first && !mbar_wait(ACC_FULL(acc.last), acc.parity(acc.last), s_abort, a.err)) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 {
-                    const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + kAccCol0 + r * kTileTok;
+                    const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + kAccCol0 + r * kTileTok + acc.first * kAccSlot;
     #pragma unroll 1
                     for (int c0 = 16 * half; c0 < cnt; c0 += kStride) {      // uniform over the warp
                         {
@@ -515,7 +564,8 @@ umma_grouped_gemm_kernel(const __grid_constant__ XMaps xmaps, const __grid_const
                     }
                 }
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                mbar_arrive(ACC_EMPTY);
+                mbar_arrive(ACC_EMPTY(acc.first));
+                if (acc.last != acc.first) mbar_arrive(ACC_EMPTY(acc.last));
             }
     
         } else {
@@ -531,9 +581,11 @@ umma_grouped_gemm_kernel(const __grid_constant__ XMaps xmaps, const __grid_const
             const int es = r + 2 * half;
             const int tid = quarter * 32 + lane;
             uint32_t unit_i = 0, stage_i = 0;
-            for (int u = blockIdx.x; u < n_units; u += gridDim.x, unit_i++) {     // (the abort flag is seen inside the wait)
+            AccCursor acc;
+            for (int u = blockIdx.x; u < n_units; u += gridDim.x, unit_i++, acc.done()) {     // (the abort flag is seen inside the wait)
                 const int4 grp = a.groups[u / n_pairs];
                 const int cnt = grp.z, pos0 = grp.y;
+                acc.take(cnt);
                 const int wrow0 = (u % n_pairs) * 2 * kTileM + r * kTileM;
                 const int wrow = wrow0 + tid;
                 const float gl = f16_global_to_f32(a.global[(size_t)grp.x * a.N + wrow]);
@@ -549,7 +601,8 @@ umma_grouped_gemm_kernel(const __grid_constant__ XMaps xmaps, const __grid_const
                 // One answer for the 128 threads of this set: they meet at named barriers below, so none may leave
                 // alone.  The same barrier publishes the factors (their buffer alternates by unit, so one barrier
                 // per unit is enough).
-                const bool mine = mbar_wait(ACC_FULL, unit_i & 1, s_abort, a.err);
+                bool mine = mbar_wait(ACC_FULL(acc.first), acc.parity(acc.first), s_abort, a.err);
+                if (mine && acc.last != acc.first) mine = mbar_wait(ACC_FULL(acc.last), acc.parity(acc.last), s_abort, a.err);
                 uint32_t all_ok;
                 asm volatile(
                     "{\n\t.reg .pred p, q;\n\t"
@@ -562,7 +615,7 @@ umma_grouped_gemm_kernel(const __grid_constant__ XMaps xmaps, const __grid_const
                 if (!all_ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 {
-                    const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + kAccCol0 + r * kTileTok;
+                    const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + kAccCol0 + r * kTileTok + acc.first * kAccSlot;
     #pragma unroll 1
                     for (int c0 = 32 * half; c0 < cnt; c0 += 64) {      // uniform over the warp
                         float v[2][16];
@@ -608,7 +661,8 @@ umma_grouped_gemm_kernel(const __grid_constant__ XMaps xmaps, const __grid_const
                     }
                 }
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                mbar_arrive(ACC_EMPTY);
+                mbar_arrive(ACC_EMPTY(acc.first));
+                if (acc.last != acc.first) mbar_arrive(ACC_EMPTY(acc.last));
             }
     
         }
@@ -851,8 +905,11 @@ int launch_prefill_umma(const BankView& b, const void* x, int x_dtype, const Dec
                                  rt.expert_ids ? &rewrite : nullptr);
     // 3. sorted, scaled f16 activations
     c.begin(K_PERMUTE_ACT);
-    prefill_gather_kernel<<<(routes + 7) / 8, 256, 0, c.s>>>(x, x_dtype, sc.route_idx, sc.seg + nbins, top_k, b.hidden, sc.xg,
-                                                   sc.row_scale);
+    // from here on every kernel is launched programmatically behind the one before (each waits for it before its first
+    // read): 2 to 3 us less between two of them
+    const int parts = std::min(top_k, tokens >= 4096 ? 1 : tokens >= 2048 ? 2 : tokens >= 1024 ? 4 : 8);
+    launch_pdl(prefill_gather_kernel, dim3((unsigned)(((size_t)tokens * parts + 7) / 8)), dim3(256), 0, c.s, x, x_dtype,
+               bins_of_route, nbins, (const int32_t*)sc.pos_of_route, tokens, top_k, parts, b.hidden, sc.xg, sc.row_scale);
     c.end();
     launches++;
 
@@ -873,10 +930,10 @@ int launch_prefill_umma(const BankView& b, const void* x, int x_dtype, const Dec
     a.global = b.gu_global; a.row_scale = sc.row_scale;
     a.ic1 = sc.ic1; a.N = 2 * b.inter;
     c.begin(K_GROUPED_GATE_UP);
-    umma_grouped_gemm_kernel<true, 2048, false><<<sm_count, kThreads, kUmmaSmemLocal, c.s>>>(map_x, map_gp, map_gs, a);
+    launch_pdl(umma_grouped_gemm_kernel<true, 2048, false>, dim3(sm_count), dim3(kThreads), kUmmaSmemLocal, c.s, map_x, map_gp, map_gs, a);
     c.end();
     c.begin(K_PREFILL_RESCALE);
-    prefill_rescale_kernel<<<(routes + 7) / 8, 256, 0, c.s>>>(sc.ic1, sc.seg + nbins, b.inter, sc.ic2h, sc.row_scale2);
+    launch_pdl(prefill_rescale_kernel, dim3((routes + 7) / 8), dim3(256), 0, c.s, sc.ic1, sc.seg + nbins, b.inter, sc.ic2h, sc.row_scale2);
     c.end();
     a.global = b.dn_global; a.row_scale = sc.row_scale2;
     a.route_weight = route_weight; a.y = sc.y; a.y_f32 = (out_dtype == 1); a.N = b.hidden;
@@ -897,7 +954,7 @@ int launch_prefill_umma(const BankView& b, const void* x, int x_dtype, const Dec
     if (ret)
         umma_grouped_gemm_kernel<false, 512, true><<<sm_count, kThreads, kUmmaSmem, c.s>>>(map_h, map_dp, map_ds, a);
     else
-        umma_grouped_gemm_kernel<false, 512, false><<<sm_count, kThreads, kUmmaSmemLocal, c.s>>>(map_h, map_dp, map_ds, a);
+        launch_pdl(umma_grouped_gemm_kernel<false, 512, false>, dim3(sm_count), dim3(kThreads), kUmmaSmemLocal, c.s, map_h, map_dp, map_ds, a);
     c.end();
     launches += 3;
     if (ret) return launches;

@@ -152,6 +152,31 @@ def test_shared_expert_on_tensor_memory_path(layer, tokens):
     assert np.abs(gate.cpu().numpy() - want_gate).max() <= 1e-5
 
 
+@pytest.mark.parametrize("tokens", [1, 8, 9, 16, 17, 32, 33, 64, 65, 130, 255])
+def test_shared_expert_token_tiles(layer, tokens):
+    """Below 256 tokens: CTAs of 8, 16, 32 and 64 tokens, either side of every step, several of the largest."""
+    test_shared_expert_on_tensor_memory_path(layer, tokens)
+
+
+@pytest.mark.parametrize("sizes", [(1, 63, 64, 65, 128, 79), (64, 64, 64, 64, 64, 80), (129, 1, 127, 2, 66, 75), (200, 16, 17, 65, 64, 38)])
+def test_passes_of_one_and_of_both_accumulator_slots(layer, sizes):
+    """Passes of up to 64 rows take one accumulator slot in turn, longer ones both: experts with row counts either side of
+    that (and of a pass of 128) in changing order.  Choice j of every token comes from experts of its own, whose row
+    counts are `sizes` rotated by j."""
+    lay, moe, banks = layer
+    n, T = len(sizes), sum(sizes)
+    ids = np.stack([j * n + np.repeat(np.roll(np.arange(n), -j), np.roll(sizes, -j)) for j in range(lay.top_k)], 1).astype(np.int32)
+    rng = np.random.default_rng(T)
+    xb = pkg.synth.make_x(7 + sizes[0], T, lay.hidden)
+    w = rng.uniform(0.05, 0.5, ids.shape).astype(np.float32)
+    got = _run(moe, lay, xb, ids, w, torch.float32, L.PATH_GROUPED)
+    want = o.grouped_moe_reference_mt(banks, lay.hidden, lay.inter, pkg.synth.bf16_bits_to_f32(xb), lay.top_k,
+                                      ids.reshape(-1), w.reshape(-1))
+    assert rel_l2(got, want) < 1e-3            # as above
+    for t in range(T):
+        assert rel_l2(got[t], want[t]) < 3e-3, t
+
+
 def test_whole_block_512_tokens_against_cpu_path(layer):
     """Router, grouped GEMM, tcgen05 shared expert and combine in one call, against the CPU checker's block."""
     lay, moe, banks = layer
