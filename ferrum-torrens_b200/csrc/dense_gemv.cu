@@ -499,19 +499,19 @@ dense_gemv_umma_kernel(const __grid_constant__ DenseMaps maps, DenseArgs a) {
     if (threadIdx.x == 0) {
         for (int s = 0; s < kUmXStages; s++) {
             mbar_init(XRAW_FULL(s), 1);
-            mbar_init(X_FULL(s), 128);
+            mbar_init(X_FULL(s), 4);
             mbar_init(X_EMPTY(s), 2);
         }
         for (int s = 0; s < kUmRawStages; s++) {
             mbar_init(RAW_FULL(s), 1);
-            mbar_init(RAW_EMPTY(s), 256);
+            mbar_init(RAW_EMPTY(s), 8);       // two pieces x four warps
         }
         for (int s = 0; s < kUmWBufs; s++) {
-            mbar_init(W_READY(s), 128);
+            mbar_init(W_READY(s), 4);
             mbar_init(W_FREE(s), 1);
         }
         mbar_init(ACC_FULL, 2);
-        mbar_init(ACC_EMPTY, 256);
+        mbar_init(ACC_EMPTY, 8);
         *s_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -666,10 +666,10 @@ dense_gemv_umma_kernel(const __grid_constant__ DenseMaps maps, DenseArgs a) {
                         h2[2 * v + 1] = __floats2half2_rn(buf[v].z * inv, buf[v].w * inv);
                     }
                     if (ks + 1 < steps) load(ks + 1);
-                    ok = mbar_wait(X_EMPTY(st), ((it / kUmXStages) & 1) ^ 1, s_abort, a.err);
+                    ok = mbar_wait_warp(X_EMPTY(st), ((it / kUmXStages) & 1) ^ 1, s_abort, a.err);
                     if (!ok) break;
                 } else {
-                    ok = mbar_wait(XRAW_FULL(st), (it / kUmXStages) & 1, s_abort, a.err);
+                    ok = mbar_wait_warp(XRAW_FULL(st), (it / kUmXStages) & 1, s_abort, a.err);
                     if (!ok) break;
                     if (in_tile) {
 #pragma unroll
@@ -692,7 +692,7 @@ dense_gemv_umma_kernel(const __grid_constant__ DenseMaps maps, DenseArgs a) {
                                        *reinterpret_cast<uint32_t*>(&h2[4 * j + 2]), *reinterpret_cast<uint32_t*>(&h2[4 * j + 3]));
                 }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");     // the tensor core reads what this thread stored
-                mbar_arrive(X_FULL(st));
+                mbar_arrive_warp(X_FULL(st));
             }
             if (!ok) break;
         }
@@ -709,7 +709,7 @@ dense_gemv_umma_kernel(const __grid_constant__ DenseMaps maps, DenseArgs a) {
                 const int c = w >> 1;
                 const uint32_t stage = stage0 + 2 * (c >> 1) + (w & 1);
                 const int st = stage % kUmRawStages;
-                ok = mbar_wait(RAW_FULL(st), (stage / kUmRawStages) & 1, s_abort, a.err);
+                ok = mbar_wait_warp(RAW_FULL(st), (stage / kUmRawStages) & 1, s_abort, a.err);
                 if (!ok) break;
                 const int wb = item % kUmWBufs;
                 const uint32_t taddr = tlane + wb * kUmWCols;
@@ -732,7 +732,7 @@ dense_gemv_umma_kernel(const __grid_constant__ DenseMaps maps, DenseArgs a) {
                 uint32_t r0[16], r1[16];
                 convert(0, r0);
                 convert(1, r1);
-                ok = mbar_wait(W_FREE(wb), ((item / kUmWBufs) & 1) ^ 1, s_abort, a.err);
+                ok = mbar_wait_warp(W_FREE(wb), ((item / kUmWBufs) & 1) ^ 1, s_abort, a.err);
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 tmem_st16(taddr, r0);
@@ -741,10 +741,10 @@ dense_gemv_umma_kernel(const __grid_constant__ DenseMaps maps, DenseArgs a) {
                 tmem_st16(taddr + 32, r0);
                 convert(3, r1);
                 tmem_st16(taddr + 48, r1);
-                mbar_arrive(RAW_EMPTY(st));
+                mbar_arrive_warp(RAW_EMPTY(st));
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                mbar_arrive(W_READY(wb));
+                mbar_arrive_warp(W_READY(wb));
             }
             if (!ok) break;
         }
@@ -755,7 +755,7 @@ dense_gemv_umma_kernel(const __grid_constant__ DenseMaps maps, DenseArgs a) {
         for (int u = blockIdx.x; u < n_units && !*s_abort; u += gridDim.x, unit_i++) {
             const int n = u * 256 + r * 128 + quarter * 32 + lane;
             const float gl = n < N ? f16_global_to_f32(a.global[n]) : 0.f;
-            if (!mbar_wait(ACC_FULL, unit_i & 1, s_abort, a.err)) break;
+            if (!mbar_wait_warp(ACC_FULL, unit_i & 1, s_abort, a.err)) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + kUmAccCol0 + r * kUmAccCols;
 #pragma unroll 1
@@ -783,7 +783,7 @@ dense_gemv_umma_kernel(const __grid_constant__ DenseMaps maps, DenseArgs a) {
                 __syncwarp();
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            mbar_arrive(ACC_EMPTY);
+            mbar_arrive_warp(ACC_EMPTY);
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
