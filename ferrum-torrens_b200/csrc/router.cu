@@ -306,6 +306,9 @@ router_fused_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __
     extern __shared__ __align__(16) uint8_t rsm[];                                        // [stages][gate rows | token rows]
     float* const slog = reinterpret_cast<float*>(rsm + kFusedStages * kFusedStageBytes);   // [tok][256], the cluster's first CTA
     pdl_launch_dependents();
+    // A CTA's shared memory may be stored to only once that CTA has started: everyone arrives here and waits in front
+    // of the remote store, where the whole k loop has hidden the wait.
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
     const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
     const int rank = (int)cluster.block_rank();   // = blockIdx.x: experts 32 * rank ..
     const int e0 = rank * 32, t0 = blockIdx.y * kFusedTok;
@@ -353,6 +356,7 @@ router_fused_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __
         }
     }
     // hand the logit to the cluster's first CTA
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");     // the first CTA is running
     float* remote = cluster.map_shared_rank(slog, 0);
     remote[warp * 256 + e0 + lane] = acc;
     cluster.sync();
