@@ -325,12 +325,8 @@ ep_dispatch_sorted_kernel(const __nv_bfloat16* __restrict__ x, const int32_t* __
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    const int ex = max((int)((__float_as_uint(m) >> 23) & 0xff), 15);
-    float inv = 1.0f, sc = 1.0f;
-    if (ex < 255) {
-        inv = __uint_as_float((uint32_t)(127 + 14 - (ex - 127)) << 23);
-        sc = __uint_as_float((uint32_t)(127 - 14 + (ex - 127)) << 23);
-    }
+    float inv, sc;
+    f16_row_scale(m, inv, sc);
     __half* const dst = reinterpret_cast<__half*>(peer_xg[p]) + (size_t)row * H;
 #pragma unroll
     for (int c = 0; c < kChunks; c++) {

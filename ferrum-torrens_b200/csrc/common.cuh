@@ -67,6 +67,18 @@ __device__ __forceinline__ void store_act(void* p, int dtype, size_t i, float v)
         reinterpret_cast<float*>(p)[i] = v;
 }
 
+// The power of two that brings a row whose largest magnitude is m into [2^14, 2^15), where an f16 keeps every bit of a bf16
+// value and eleven of an f32 one, and its reciprocal (both exact).  Magnitudes below 2^-112 would need a factor past the
+// largest float: such rows take the factor of 2^-112 and stay exact all the same.  Rows with an infinity stay as they are.
+__device__ __forceinline__ void f16_row_scale(float m, float& inv, float& sc) {
+    const uint32_t e = max((__float_as_uint(m) >> 23) & 0xffu, 15u);
+    inv = sc = 1.0f;
+    if (e < 255) {
+        inv = __uint_as_float((127 + 14 + 127 - e) << 23);
+        sc = __uint_as_float((e - 14) << 23);
+    }
+}
+
 // device view of the six banks plus the shapes the kernels index with
 struct BankView {
     const uint8_t* gu_packed;  // [slots, 2I, H/2]

@@ -339,14 +339,8 @@ __device__ __forceinline__ void convert_group_tokens(const ExpertArgs& a, const 
             for (int q = 0; q < 8; q++) m = fmaxf(m, fabsf(v[c8][q]));
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-        // largest magnitude into [2^14, 2^15): exact power-of-two scaling, f16 keeps every bit of
-        // a bf16 input and 11 bits of an f32 one
-        const int e = (int)((__float_as_uint(m) >> 23) & 0xff);
-        float inv = 1.0f, sc = 1.0f;
-        if (e > 0 && e < 255) {
-            inv = __uint_as_float((uint32_t)(127 + 14 - (e - 127)) << 23);
-            sc = __uint_as_float((uint32_t)(127 - 14 + (e - 127)) << 23);
-        }
+        float inv, sc;
+        f16_row_scale(m, inv, sc);
         __half* xrow = reinterpret_cast<__half*>(xtile + (size_t)tk * RSX);
 #pragma unroll
         for (int c8 = 0; c8 < K / 256; c8++) {

@@ -104,13 +104,8 @@ __global__ void __launch_bounds__(kDgWarps * 32, 2) dense_gemv_kernel(DenseArgs 
         for (int k = lane; k < K; k += 32) m = fmaxf(m, fabsf(load_act(a.a, a.a_dtype, row + k)));
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-        // largest magnitude into [2^14, 2^15): exact power-of-two scaling into the f16 range
-        const int e = (int)((__float_as_uint(m) >> 23) & 0xff);
-        float inv = 1.0f, sc = 1.0f;
-        if (e > 0 && e < 255) {
-            inv = __uint_as_float((uint32_t)(127 + 14 - (e - 127)) << 23);
-            sc = __uint_as_float((uint32_t)(127 - 14 + (e - 127)) << 23);
-        }
+        float inv, sc;
+        f16_row_scale(m, inv, sc);
         for (int k = lane * 2; k < K; k += 64) {
             const float v0 = load_act(a.a, a.a_dtype, row + k), v1 = load_act(a.a, a.a_dtype, row + k + 1);
             *reinterpret_cast<__half2*>(xrow + k) = __floats2half2_rn(v0 * inv, v1 * inv);
@@ -327,12 +322,8 @@ dense_gemv_tma_kernel(const __grid_constant__ DenseMaps maps, DenseArgs a) {
         for (int k = lane; k < K; k += 32) m = fmaxf(m, fabsf(load_act(a.a, a.a_dtype, row + k)));
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-        const int e = (int)((__float_as_uint(m) >> 23) & 0xff);
-        float inv = 1.0f, sc = 1.0f;
-        if (e > 0 && e < 255) {
-            inv = __uint_as_float((uint32_t)(127 + 14 - (e - 127)) << 23);
-            sc = __uint_as_float((uint32_t)(127 - 14 + (e - 127)) << 23);
-        }
+        float inv, sc;
+        f16_row_scale(m, inv, sc);
 #pragma unroll 8
         for (int k = lane * 2; k < K; k += 64) {
             const float v0 = load_act(a.a, a.a_dtype, row + k), v1 = load_act(a.a, a.a_dtype, row + k + 1);
@@ -552,9 +543,9 @@ dense_gemv_umma_kernel(const __grid_constant__ DenseMaps maps, DenseArgs a) {
             }
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-            // (exponents below 15 would need a factor past the largest float: such rows keep 15's, exact all the same)
-            const int e = max((int)((__float_as_uint(m) >> 23) & 0xff), 15);
-            if (lane == 0) s_scale[tk] = e < 255 ? __uint_as_float((uint32_t)(127 - 14 + (e - 127)) << 23) : 1.0f;
+            float inv, sc;
+            f16_row_scale(m, inv, sc);
+            if (lane == 0) s_scale[tk] = sc;
         }
         asm volatile("bar.sync 1, %0;" ::"n"(kUmThreads - 32) : "memory");
     }

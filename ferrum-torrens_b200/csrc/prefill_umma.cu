@@ -125,13 +125,8 @@ prefill_gather_kernel(const void* __restrict__ x, int x_dtype, const int32_t* __
         for (int q = 0; q < 8; q++) m = fmaxf(m, fabsf(v[c][q]));
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    // largest magnitude into [2^14, 2^15): exact power-of-two scaling
-    const int e = max((int)((__float_as_uint(m) >> 23) & 0xff), 15);
-    float inv = 1.0f, sc = 1.0f;
-    if (e < 255) {
-        inv = __uint_as_float((uint32_t)(127 + 14 - (e - 127)) << 23);
-        sc = __uint_as_float((uint32_t)(127 - 14 + (e - 127)) << 23);
-    }
+    float inv, sc;
+    f16_row_scale(m, inv, sc);
     __half2 h[kChunksPerLane][4];
 #pragma unroll
     for (int c = 0; c < kChunksPerLane; c++)
@@ -179,12 +174,8 @@ prefill_rescale_kernel(const float* __restrict__ ic1, const int32_t* __restrict_
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    const int e = max((int)((__float_as_uint(m) >> 23) & 0xff), 15);
-    float inv = 1.0f, sc = 1.0f;
-    if (e < 255) {
-        inv = __uint_as_float((uint32_t)(127 + 14 - (e - 127)) << 23);
-        sc = __uint_as_float((uint32_t)(127 - 14 + (e - 127)) << 23);
-    }
+    float inv, sc;
+    f16_row_scale(m, inv, sc);
 #pragma unroll
     for (int c = 0; c < 2; c++) {
         __half2 h[4];

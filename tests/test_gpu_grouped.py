@@ -177,6 +177,27 @@ def test_passes_of_one_and_of_both_accumulator_slots(layer, sizes):
         assert rel_l2(got[t], want[t]) < 3e-3, t
 
 
+@pytest.mark.parametrize("path", [L.PATH_GEMV, L.PATH_GROUPED])
+def test_rows_of_every_size(layer, path):
+    """Rows from 2^-125 to 2^0: a row of x below 2^-112, or one of the intermediate (about the square of x), would need a
+    scaling factor past the largest float.  Where the exact result is a normal float the bar is the usual one (f16 keeps
+    eleven bits of the intermediate's largest values); below, the result's own spacing 2^-149 comes on top."""
+    lay, moe, banks = layer
+    rng = np.random.default_rng(3)
+    size = [0, 20, 50, 52, 53, 54, 55, 56, 57, 58, 59, 60, 61, 62, 64, 90, 110, 112, 113, 114, 118, 122, 125]
+    x = pkg.synth.bf16_bits_to_f32(pkg.synth.make_x(9, len(size), lay.hidden))
+    x = (x * 2.0 ** -np.array(size, np.float64)[:, None]).astype(np.float32)
+    xb = (x.view(np.uint32) >> 16).astype(np.uint16)       # (bf16 rounds its own subnormals)
+    ids = _ids(rng, len(size), lay.experts, lay.top_k)
+    w = rng.uniform(0.05, 0.5, ids.shape).astype(np.float32)
+    got = _run(moe, lay, xb, ids, w, torch.float32, path).astype(np.float64)
+    want = o.grouped_moe_reference_mt(banks, lay.hidden, lay.inter, pkg.synth.bf16_bits_to_f32(xb), lay.top_k,
+                                      ids.reshape(-1), w.reshape(-1)).astype(np.float64)
+    assert np.isfinite(got).all()
+    for t in range(len(size)):
+        assert np.linalg.norm(got[t] - want[t]) <= 3e-3 * np.linalg.norm(want[t]) + 2.0 ** -149 * lay.top_k * lay.hidden ** 0.5, size[t]
+
+
 def test_whole_block_512_tokens_against_cpu_path(layer):
     """Router, grouped GEMM, tcgen05 shared expert and combine in one call, against the CPU checker's block."""
     lay, moe, banks = layer

@@ -254,6 +254,30 @@ def test_dense_gemv_many_tokens_against_cpu_path(m, n, k, dtype):
     moe.close()
 
 
+@pytest.mark.parametrize("m,n,k", [(1, 36, 64), (9, 260, 512), (3, 1056, 512), (9, 1056, 512), (17, 1056, 512), (65, 1056, 512)])
+def test_dense_gemv_of_tiny_rows(m, n, k):
+    """Rows around 2^-112 .. 2^-124, whose scaling into the f16 range would need a factor past the largest float: the
+    register-streaming kernel, the TMA-fed one (one and two token tiles), the tensor-memory kernel, and its remainder.
+    The globals are 2^0, so that most results are normal floats; besides the usual bar, each of the two partial sums of a
+    row may lose what lies below 2^-126 (an f32 atomic add flushes subnormals to zero)."""
+    a, pk, sk, _ = _gemv_case(m, n, k, 5000 + m + n)
+    x = o.bf16_bits_to_f32(a).copy()
+    x *= 2.0 ** -np.ceil(np.log2(np.abs(x).max(1, keepdims=True)))
+    x[m - 1] *= 2.0 ** -120
+    if m > 1:
+        x[0], x[1] = x[0] * 2.0 ** -113, x[1] * 2.0 ** -116
+    bits = (x.view(np.uint32) >> 16).astype(np.uint16)
+    x = o.bf16_bits_to_f32(bits)               # (a bf16 below 2^-126 has fewer bits)
+    glob = np.ones(n, np.float16)
+    moe = tiny_handle(64)
+    got = _run_gemv(moe, bits, pk, sk, glob)
+    moe.sync_status()
+    want = o.nvfp4_dense_gemv(x, pk, sk, glob.view(np.uint16))
+    for i in range(m):
+        assert np.linalg.norm(got[i].astype(np.float64) - want[i]) <= 1e-5 * np.linalg.norm(want[i].astype(np.float64)) + 2.0 ** -125 * n ** 0.5, i
+    moe.close()
+
+
 def test_dense_gemv_rejects_shapes_it_was_not_built_for():
     moe = tiny_handle(64)
     a, pk, sk, glob = _gemv_case(1, 8, 64, 5)
