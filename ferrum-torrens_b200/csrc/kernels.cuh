@@ -46,7 +46,9 @@ struct Ctx {
 
 // Programmatic dependent launch for chains of small dependent kernels (the decode step): the next kernel of the
 // stream may be scheduled while its predecessor drains; it calls pdl_wait() before it reads what the
-// predecessor wrote.  Both calls are no-ops for a kernel launched the ordinary way.
+// predecessor wrote.  Both calls are no-ops for a kernel launched the ordinary way.  Such a kernel's pointers to what
+// the predecessor writes are not `const .. __restrict__`: that would promise data no one writes while the kernel runs, and
+// allow reads in front of the wait or through the read-only path.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

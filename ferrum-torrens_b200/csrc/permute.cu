@@ -47,7 +47,7 @@ __device__ __forceinline__ void count_chunk(const int32_t* route_bin, int routes
 }
 
 // stable scatter of this CTA's chunk; wbase[w][b] = first output position of warp w's routes of bin b
-__device__ __forceinline__ void scatter_chunk(const int32_t* __restrict__ route_bin, int routes, int bins,
+__device__ __forceinline__ void scatter_chunk(const int32_t* route_bin, int routes, int bins,
                                               int chunk_begin, int warp_routes, int* wbase, int32_t* __restrict__ route_idx,
                                               int32_t* __restrict__ pos_of_route) {
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
@@ -173,7 +173,7 @@ csr_count_kernel(const int32_t* route_bin, int routes, int bins, int chunk, int3
 // groups_from_csr_kernel does in a launch of its own): (slot, first sorted row, rows, 0) per pass, bins whose slot
 // is not resident skipped, the number of passes in *g.n_groups.
 __global__ void __launch_bounds__(kMaxBins)
-csr_scan_kernel(int32_t* __restrict__ cta_hist, int nctas, int bins, int32_t* __restrict__ seg, CsrGroups g) {
+csr_scan_kernel(int32_t* cta_hist, int nctas, int bins, int32_t* __restrict__ seg, CsrGroups g) {
     __shared__ int wsum[32];
     const int b = threadIdx.x;
     pdl_launch_dependents();
@@ -248,8 +248,8 @@ csr_scan_kernel(int32_t* __restrict__ cta_hist, int nctas, int bins, int32_t* __
 
 // pass 3: recount per warp, then ranked scatter from the CTA's bases
 __global__ void __launch_bounds__(kThreads)
-csr_scatter_kernel(const int32_t* __restrict__ route_bin, int routes, int bins, int chunk,
-                   const int32_t* __restrict__ cta_base, int32_t* __restrict__ route_idx, int32_t* scratch_flag,
+csr_scatter_kernel(const int32_t* route_bin, int routes, int bins, int chunk,
+                   const int32_t* cta_base, int32_t* __restrict__ route_idx, int32_t* scratch_flag,
                    int32_t* __restrict__ pos_of_route) {
     extern __shared__ int sm[];
     pdl_launch_dependents();

@@ -83,8 +83,8 @@ __device__ __forceinline__ uint32_t hmul2_f16(uint32_t a, uint32_t b) {
 // the writes (top_k rows of 4 KB per token): one warp per sorted row read and converted every row top_k times (8192
 // tokens: 60 us).  Small batches cut a token's routes into parts to have warps for every SM.
 __global__ void __launch_bounds__(256)
-prefill_gather_kernel(const void* __restrict__ x, int x_dtype, const int32_t* __restrict__ bin_of_route, int nbins,
-                      const int32_t* __restrict__ pos_of_route, int tokens, int top_k, int parts, int K, __half* __restrict__ xg,
+prefill_gather_kernel(const void* x, int x_dtype, const int32_t* bin_of_route, int nbins,
+                      const int32_t* pos_of_route, int tokens, int top_k, int parts, int K, __half* __restrict__ xg,
                       float* __restrict__ row_scale) {
     const int w = blockIdx.x * 8 + threadIdx.x / 32, lane = threadIdx.x % 32;
     const int t = w / parts, part = w % parts;
@@ -148,7 +148,7 @@ prefill_gather_kernel(const void* __restrict__ x, int x_dtype, const int32_t* __
 // ic1 (f32, sorted rows: gate | up) -> ic2 = silu(gate) * up as f16 with a per-row power-of-two scale.
 // One warp per row; K == 512.
 __global__ void __launch_bounds__(256)
-prefill_rescale_kernel(const float* __restrict__ ic1, const int32_t* __restrict__ n_sorted, int K,
+prefill_rescale_kernel(const float* ic1, const int32_t* n_sorted, int K,
                        __half* __restrict__ ic2h, float* __restrict__ row_scale) {
     const int row = blockIdx.x * 8 + threadIdx.x / 32, lane = threadIdx.x % 32;
     pdl_launch_dependents();

@@ -134,7 +134,7 @@ __device__ __forceinline__ void load_rows(uint4 (&lo)[SB], uint4 (&hi)[SB], cons
         }
 }
 template <int NT, int SB, int UB>
-__device__ __forceinline__ void mma_rows(const uint4 (&lo)[SB], const uint4 (&hi)[SB], const __nv_bfloat16* __restrict__ x,
+__device__ __forceinline__ void mma_rows(const uint4 (&lo)[SB], const uint4 (&hi)[SB], const __nv_bfloat16* x,
                                          int ldx, int tok0, int tokens, int k, int k_end, int g8, float (&acc)[NT][4]) {
     const uint4 zero = make_uint4(0, 0, 0, 0);
 #pragma unroll
@@ -239,7 +239,7 @@ shared_phase1_mma_kernel(const __nv_bfloat16* __restrict__ x, int tokens, int H,
 // launch: the weight rows (which phase 1 does not write) are asked for before its result is waited for.
 template <int NT>
 __global__ void __launch_bounds__(64)
-shared_phase2_mma_kernel(const __nv_bfloat16* __restrict__ ic2b, int tokens, int H, int SI,
+shared_phase2_mma_kernel(const __nv_bfloat16* ic2b, int tokens, int H, int SI,
                          const __nv_bfloat16* __restrict__ down, float* __restrict__ shared_out) {
     constexpr int SB = NT == 8 ? 4 : 8, UB = NT == 8 ? 1 : NT == 4 ? 2 : 4;
     __shared__ float red[NT][32][4];

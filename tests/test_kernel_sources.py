@@ -38,3 +38,19 @@ def test_remote_shared_memory_is_stored_to_after_a_cluster_barrier():
         assert "barrier.cluster.wait" in before or "cluster.sync()" in before, (path, name)
         assert "barrier.cluster.wait" not in before or "barrier.cluster.arrive" in before[:before.index("barrier.cluster.wait")], (path, name)
     assert found
+
+
+def test_overlapped_kernels_promise_no_read_only_data_but_weights():
+    """A kernel launched programmatically is resident while its predecessor still writes: `const .. __restrict__` on such
+    data would let the compiler read it before the dependency wait.  Weights are constant all the same."""
+    weights = {"gate_up", "down", "shared_gate", "gate_w"}
+    launched = set()
+    for path in glob.glob(os.path.join(CSRC, "*.cu")):
+        launched |= set(re.findall(r"launch_pdl\(\s*(\w+_kernel)", open(path).read()))
+    assert launched
+    for path, name, params, body in _kernels():
+        if name not in launched:
+            continue
+        bad = set(re.findall(r"const\s+[\w:]+\s*\*\s*__restrict__\s+(\w+)", params)) - weights
+        assert not bad, (path, name, bad)
+        assert "pdl_wait()" in body, (path, name)
