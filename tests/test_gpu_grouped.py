@@ -154,7 +154,7 @@ def test_shared_expert_on_tensor_memory_path(layer, tokens):
 
 @pytest.mark.parametrize("tokens", [1, 8, 9, 16, 17, 32, 33, 64, 65, 130, 255])
 def test_shared_expert_token_tiles(layer, tokens):
-    """Below 256 tokens: CTAs of 8, 16, 32 and 64 tokens, either side of every step, several of the largest."""
+    """Below 256 tokens: CTAs of 8, 16 and 64 tokens, either side of every step, several of the largest."""
     test_shared_expert_on_tensor_memory_path(layer, tokens)
 
 
