@@ -160,11 +160,12 @@ __device__ __forceinline__ void mma_rows(const uint4 (&lo)[SB], const uint4 (&hi
     }
 }
 
-// phase 1: grid (SI / 8, ceil(T / (8 * NT))); 8 warps split K; rows = 8 gate rows + the 8 matching up rows.  A ninth warp
-// produces the sigmoid gates: token i of the tile belongs to the CTA with blockIdx.x = i % gridDim.x (the first CTA
-// used to do all of them, after its rows, and every other CTA waited for it).
+// phase 1: grid (SI / 8 + NT, ceil(T / (8 * NT))); 8 warps split K; rows = 8 gate rows + the 8 matching up rows.  The last NT
+// CTAs of a token tile produce its sigmoid gates, one token per warp.  (A ninth warp of every CTA did them: 288 threads of
+// 130 registers leave one CTA per SM, and from 129 tokens on a router beside it waited for a second round.  Eight warps
+// of at most 128 registers are two CTAs per SM.)
 template <int NT>
-__global__ void __launch_bounds__(288)
+__global__ void __launch_bounds__(256, 2)
 shared_phase1_mma_kernel(const __nv_bfloat16* __restrict__ x, int tokens, int H, int SI,
                          const __nv_bfloat16* __restrict__ gate_up, const __nv_bfloat16* __restrict__ shared_gate,
                          __nv_bfloat16* __restrict__ ic2b, float* __restrict__ se_gate) {
@@ -174,42 +175,40 @@ shared_phase1_mma_kernel(const __nv_bfloat16* __restrict__ x, int tokens, int H,
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const int g8 = lane >> 2, t4 = lane & 3;
     const int pair0 = blockIdx.x * 8, tok0 = blockIdx.y * (8 * NT);
-    if (warp < 8) {
-        const int kper = H / 8, k_end = (warp + 1) * kper;
-        const __nv_bfloat16 *w_lo = gate_up + (size_t)(pair0 + g8) * H, *w_hi = gate_up + (size_t)(SI + pair0 + g8) * H;
-        float acc[NT][4];
-#pragma unroll
-        for (int n = 0; n < NT; n++)
-#pragma unroll
-            for (int q = 0; q < 4; q++) acc[n][q] = 0.f;
-        for (int k = warp * kper + t4 * 8; k < k_end; k += SB * 32) {
-            uint4 lo[SB], hi[SB];
-            load_rows<NT, SB, UB>(lo, hi, w_lo, w_hi, k, k_end);
-            mma_rows<NT, SB, UB>(lo, hi, x, H, tok0, tokens, k, k_end, g8, acc);
-        }
-#pragma unroll
-        for (int n = 0; n < NT; n++)
-            *reinterpret_cast<float4*>(red[warp][n][lane]) = make_float4(acc[n][0], acc[n][1], acc[n][2], acc[n][3]);
-    } else {
-        for (int tl = blockIdx.x; tl < 8 * NT; tl += gridDim.x) {
-            const int t = tok0 + tl;
-            if (t >= tokens) break;
-            float a = 0.f;
+    if (blockIdx.x >= SI / 8) {
+        const int t = tok0 + (blockIdx.x - SI / 8) * 8 + warp;
+        if (t >= tokens) return;
+        float a = 0.f;
 #pragma unroll 8
-            for (int k = lane * 8; k < H; k += 256) {
-                const uint4 wv = *reinterpret_cast<const uint4*>(shared_gate + k);
-                const uint4 xv = *reinterpret_cast<const uint4*>(x + (size_t)t * H + k);
-                const uint32_t ww[4] = {wv.x, wv.y, wv.z, wv.w}, xx[4] = {xv.x, xv.y, xv.z, xv.w};
+        for (int k = lane * 8; k < H; k += 256) {
+            const uint4 wv = *reinterpret_cast<const uint4*>(shared_gate + k);
+            const uint4 xv = *reinterpret_cast<const uint4*>(x + (size_t)t * H + k);
+            const uint32_t ww[4] = {wv.x, wv.y, wv.z, wv.w}, xx[4] = {xv.x, xv.y, xv.z, xv.w};
 #pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    const float2 w2 = bf16x2_to_f32(ww[q]), x2 = bf16x2_to_f32(xx[q]);
-                    a += w2.x * x2.x + w2.y * x2.y;
-                }
+            for (int q = 0; q < 4; q++) {
+                const float2 w2 = bf16x2_to_f32(ww[q]), x2 = bf16x2_to_f32(xx[q]);
+                a += w2.x * x2.x + w2.y * x2.y;
             }
-            a = warp_sum(a);
-            if (lane == 0) se_gate[t] = 1.0f / (1.0f + expf(-a));
         }
+        a = warp_sum(a);
+        if (lane == 0) se_gate[t] = 1.0f / (1.0f + expf(-a));
+        return;
     }
+    const int kper = H / 8, k_end = (warp + 1) * kper;
+    const __nv_bfloat16 *w_lo = gate_up + (size_t)(pair0 + g8) * H, *w_hi = gate_up + (size_t)(SI + pair0 + g8) * H;
+    float acc[NT][4];
+#pragma unroll
+    for (int n = 0; n < NT; n++)
+#pragma unroll
+        for (int q = 0; q < 4; q++) acc[n][q] = 0.f;
+    for (int k = warp * kper + t4 * 8; k < k_end; k += SB * 32) {
+        uint4 lo[SB], hi[SB];
+        load_rows<NT, SB, UB>(lo, hi, w_lo, w_hi, k, k_end);
+        mma_rows<NT, SB, UB>(lo, hi, x, H, tok0, tokens, k, k_end, g8, acc);
+    }
+#pragma unroll
+    for (int n = 0; n < NT; n++)
+        *reinterpret_cast<float4*>(red[warp][n][lane]) = make_float4(acc[n][0], acc[n][1], acc[n][2], acc[n][3]);
     __syncthreads();
     // warp n finishes token tile n: sum the K partials, silu(gate) * up
     if (warp < NT) {
@@ -291,7 +290,7 @@ void launch_mma(const __nv_bfloat16* x, int tokens, int H, int SI, const __nv_bf
                 const __nv_bfloat16* shared_gate, __nv_bfloat16* ic2b, float* shared_out, float* se_gate, const Ctx& c) {
     const int tiles = (tokens + 8 * NT - 1) / (8 * NT);
     c.begin(K_SHARED_PHASE1);
-    shared_phase1_mma_kernel<NT><<<dim3(SI / 8, tiles), 288, 0, c.s>>>(x, tokens, H, SI, gate_up, shared_gate, ic2b, se_gate);
+    shared_phase1_mma_kernel<NT><<<dim3(SI / 8 + NT, tiles), 256, 0, c.s>>>(x, tokens, H, SI, gate_up, shared_gate, ic2b, se_gate);
     c.end();
     c.begin(K_SHARED_PHASE2);
     launch_pdl(shared_phase2_mma_kernel<NT>, dim3(H / 16, tiles), dim3(64), 0, c.s, (const __nv_bfloat16*)ic2b, tokens, H, SI, down,
