@@ -100,6 +100,7 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
 // two 31.5); one expert per lane is for the batches whose 32-expert tiles are at most one per SM (256 tokens 25.6 us, with two 31.3).  Packing two chains into fma.rn.f32x2 brought nothing: it issues at less than half the rate of the scalar fma.
 constexpr int kNT = 4, kNK = 128;
 constexpr int kNTok = 4 * kNT;
+constexpr size_t kOneCtaSmem = 116 * 1024;  // of 228 KB
 constexpr int kNWStride = kNK * 2 + 16;     // bytes per expert row in shared memory (conflict-free 128-bit reads)
 
 template <int kNE>
@@ -581,10 +582,15 @@ router_logits_big_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat1
 template <int NE>
 void launch_narrow(const __nv_bfloat16* x, const __nv_bfloat16* gate_w, int tokens, int experts, int hidden, float* logits,
                    const Ctx& c) {
-    constexpr size_t smem = 2 * 32 * NE * kNWStride + 2 * kNK * kNTok * sizeof(float);
+    // One expert per lane is for batches with at most one tile per SM.  Beside the first phase of the shared expert's
+    // mma.sync kernels (fewer than 256 tokens) its CTAs would pile up on the SMs that come free first (200 tokens in a
+    // graph: 81 us instead of 23), so they ask for more than half of an SM's shared memory.  Beside the tcgen05 kernels, whose
+    // CTAs leave no room for that, they do not.
+    constexpr size_t need = 2 * 32 * NE * kNWStride + 2 * kNK * kNTok * sizeof(float);
+    const size_t smem = NE == 1 && tokens < 256 ? kOneCtaSmem : need;
     const dim3 grid((experts + 32 * NE - 1) / (32 * NE), (tokens + kNTok - 1) / kNTok);
     static PerDeviceOnce once;
-    allow_dyn_smem(once, router_logits_narrow_kernel<NE>, smem);
+    allow_dyn_smem(once, router_logits_narrow_kernel<NE>, NE == 1 ? kOneCtaSmem : need);
     c.begin(K_ROUTER_LOGITS);
     router_logits_narrow_kernel<NE><<<grid, 128, smem, c.s>>>(x, gate_w, tokens, experts, hidden, logits);
     c.end();
