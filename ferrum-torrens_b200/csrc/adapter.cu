@@ -306,7 +306,11 @@ int run_routed(ftm_handle* h, const void* x, int x_dtype, const void* expert_ids
                          h->route_expert, h->seg, h->csr_scratch, h->flags + 3};
         DecodeRoutes rt{expert_ids ? nullptr : h->route_slot, expert_ids, ids_dtype, layer, h->cfg.experts,
                         (int)h->slot_for_id.size(), h->d_slot_for_id, h->route_slot, h->flags + 1};
-        h->launches += launch_decode_mma(b, x, x_dtype, rt, weights, tokens, h->cfg.top_k, sc, h->sm_count, h->ctx(s));
+        // Beside the tcgen05 shared expert gate_up waits for it: its CTAs would otherwise settle on the SMs that kernel has
+        // not taken and stay there, uneven (a block of 256 tokens 246 us, 186 with the wait; 176 and 147 under skewed routing).
+        // The mma.sync shared expert of smaller batches leaves room on every SM and is not waited for.
+        const cudaEvent_t before = join && shared_umma_supported(tokens, h->cfg.hidden, h->cfg.shared_inter) ? join : nullptr;
+        h->launches += launch_decode_mma(b, x, x_dtype, rt, weights, tokens, h->cfg.top_k, sc, h->sm_count, before, h->ctx(s));
     } else {
         const __nv_bfloat16* xb = nullptr;
         int rc = stage_x(h, x, x_dtype, tokens, &xb, s);

@@ -1035,7 +1035,7 @@ bool decode_mma_supported(int hidden, int inter, int routes, int slots, int expe
 
 int launch_decode_mma(const BankView& b, const void* x, int x_dtype, const DecodeRoutes& rt,
                       const float* route_weight, int tokens, int top_k, DecodeScratch sc, int sm_count,
-                      const Ctx& c) {
+                      cudaEvent_t before_experts, const Ctx& c) {
     const int routes = tokens * top_k;
     const bool small = routes <= kPlanMaxRoutes;
     int launches = 0;
@@ -1087,6 +1087,7 @@ int launch_decode_mma(const BankView& b, const void* x, int x_dtype, const Decod
     // gate_up: K = hidden, N = 2 * inter rows
     a.packed = b.gu_packed; a.scale = b.gu_scale; a.scale_frag = b.gu_scale_frag; a.global = b.gu_global;
     a.act = x; a.act_dtype = x_dtype; a.ic2 = sc.ic2p; a.N = 2 * b.inter;
+    if (small && before_experts) cudaStreamWaitEvent(c.s, before_experts, 0);
     c.begin(K_EXPERT_GATE_UP);
     if (small)
         launch_expert<true, 2048, 1, 1>(a, sm_count, c.s, true);

@@ -158,7 +158,7 @@ struct DecodeRoutes {
 bool decode_mma_supported(int hidden, int inter, int routes, int slots, int experts, bool have_expert_ids);
 int launch_decode_mma(const BankView& b, const void* x, int x_dtype, const DecodeRoutes& rt,
                       const float* route_weight, int tokens, int top_k, DecodeScratch sc, int sm_count,
-                      const Ctx& c);
+                      cudaEvent_t before_experts /* gate_up of a plan's step waits for it; or null */, const Ctx& c);
 
 // fragment-ordered copy of one slot's block scales (both projections), after the slot's bytes have landed
 int launch_scale_repack(const BankView& b, int slot, uint8_t* gu_scale_frag, uint8_t* dn_scale_frag, const Ctx& c);
