@@ -177,6 +177,19 @@ def test_passes_of_one_and_of_both_accumulator_slots(layer, sizes):
         assert rel_l2(got[t], want[t]) < 3e-3, t
 
 
+@pytest.mark.parametrize("sms", [1, 3, 16])
+def test_long_and_short_passes_in_every_order_on_few_ctas(layer, sms):
+    """The same on a few CTAs, each of which walks dozens to hundreds of units: long and short passes follow one another in
+    every order, so that every rule of which accumulator slot waits for which is met."""
+    _, moe, _ = layer
+    moe.set_sm_budget(sms)
+    try:
+        for sizes in ((129, 1, 127, 2, 66, 75), (65, 200, 5, 90, 16, 64)):
+            test_passes_of_one_and_of_both_accumulator_slots(layer, sizes)
+    finally:
+        moe.set_sm_budget(0)
+
+
 @pytest.mark.parametrize("path", [L.PATH_GEMV, L.PATH_GROUPED])
 def test_rows_of_every_size(layer, path):
     """Rows from 2^-125 to 2^0: a row of x below 2^-112, or one of the intermediate (about the square of x), would need a
