@@ -270,7 +270,6 @@ umma_grouped_gemm_kernel(const __grid_constant__ XMaps xmaps, const __grid_const
     constexpr int kRS = RET ? kRawStages - 1 : kRawStages;   // the owner's variant gives a raw stage to its epilogue staging
     constexpr int kWarpEpi2 = kWarpDeq0 + 4 * kDeqSets;     // down: warps 16..19 row tile 0, 20..23 row tile 1
     extern __shared__ uint8_t smem_raw[];
-    pdl_launch_dependents();
     // 1024-byte alignment for the swizzled tiles
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     uint8_t* const x_tiles = smem;                                         // [kXStages][16 KiB]: 128 tokens x 64 k
@@ -1001,8 +1000,9 @@ int launch_prefill_umma_presorted(const BankView& b, const float* row_scale, con
     a.groups = sc.groups; a.n_groups = sc.n_groups; a.route_idx = nullptr; a.err = sc.err;
     a.global = b.gu_global; a.row_scale = row_scale;
     a.ic1 = sc.ic1; a.N = 2 * b.inter;
+    // (both GEMMs chained as in the path above: 4096 / 8192 tokens 382.6 / 651.4 us without, 374.3 / 636.8 with)
     c.begin(K_GROUPED_GATE_UP);
-    umma_grouped_gemm_kernel<true, 2048, false><<<sm_count, kThreads, kUmmaSmemLocal, c.s>>>(map_x, maps.gp, maps.gs, a);
+    launch_pdl(umma_grouped_gemm_kernel<true, 2048, false>, dim3(sm_count), dim3(kThreads), kUmmaSmemLocal, c.s, map_x, maps.gp, maps.gs, a);
     c.end();
     c.begin(K_PREFILL_RESCALE);
     prefill_rescale_kernel<<<(rows + 7) / 8, 256, 0, c.s>>>(sc.ic1, sc.seg + per, b.inter, sc.ic2h, sc.row_scale2);
@@ -1010,7 +1010,7 @@ int launch_prefill_umma_presorted(const BankView& b, const float* row_scale, con
     a.global = b.dn_global; a.row_scale = sc.row_scale2;
     a.route_weight = route_weight; a.y = nullptr; a.y_f32 = 0; a.N = b.hidden; a.row_dest = row_dest;
     c.begin(K_GROUPED_DOWN);
-    umma_grouped_gemm_kernel<false, 512, true><<<sm_count, kThreads, kUmmaSmem, c.s>>>(map_h, maps.dp, maps.ds, a);
+    launch_pdl(umma_grouped_gemm_kernel<false, 512, true>, dim3(sm_count), dim3(kThreads), kUmmaSmem, c.s, map_h, maps.dp, maps.ds, a);
     c.end();
     return launches + 3;
 }
