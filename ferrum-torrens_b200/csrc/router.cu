@@ -654,9 +654,10 @@ int launch_router_logits(const __nv_bfloat16* x, const __nv_bfloat16* gate_w, in
 }
 
 bool router_fused_supported(int tokens, int experts, int hidden, int top_k) {
-    // router alone: 128 tokens 15.6 us, 173 tokens 21.4, 200 tokens 27.0 here; 25.5 from 1 to 288 tokens with the narrow
-    // kernel and the separate top-k.  The cluster kernel re-reads the gate weight once per four tokens.
-    return experts == 256 && hidden % 256 == 0 && tokens < 192 && top_k <= 32;
+    // router alone: 128 tokens 15.6 us, 173 and 192 tokens 21.3, 193 tokens 26.5 here; 25.9 at 192 and 26.0 from 193 to 288
+    // tokens with the narrow kernel and the separate top-k (23.6 at 192 before either).  The cluster kernel re-reads the gate
+    // weight once per four tokens.
+    return experts == 256 && hidden % 256 == 0 && tokens <= 192 && top_k <= 32;
 }
 
 int launch_router_fused(const __nv_bfloat16* x, const __nv_bfloat16* gate_w, int tokens, int hidden, int top_k,
