@@ -1240,6 +1240,9 @@ FTM_API int ftm_dense_gemv(ftm_handle* h, const void* a, int a_dtype, const void
     if (m <= 0 || n <= 0 || k <= 0) return fail(h, FTM_ERR_BAD, shapes, "a = [M, K] and packed = [K // 8, N]");
     if (!dense_gemv_supported(n, k))
         return fail(h, FTM_ERR_BAD, shapes, "N a multiple of 4 and K a multiple of 32 (at most 3136)");
+    // four rows of a k-word are one 128-bit load, their block scales one 32-bit load: anything less aligned would fault
+    if ((reinterpret_cast<uintptr_t>(packed_kmajor_i32) & 15) || (reinterpret_cast<uintptr_t>(scale_kmajor_u8) & 3))
+        return fail(h, FTM_ERR_BAD, "moe: dense gemv: packed must be 16-byte aligned and scale 4-byte aligned");
     h->launches += launch_dense_gemv(a, a_dtype, (const uint32_t*)packed_kmajor_i32, (const uint8_t*)scale_kmajor_u8,
                                      (const uint16_t*)global_f16, m, n, k, c, h->sm_count, h->flags + 2, h->ctx(pick(h, stream)));
     CU(h, cudaGetLastError());

@@ -250,8 +250,10 @@ FTM_API int ftm_moe_block_prenorm(ftm_handle* h, int32_t layer, const void* attn
  * c = a @ dequant(packed, scale, global)^T for the lm_head.  a [M, K] bf16 or f32 dev; the weight is the
  * engine's K-major resident bank: packed [K/8, N] int32 (word (w, n) = the eight e2m1 codes k = 8w .. 8w+7
  * of row n, nibble j -> k = 8w + j), scale [K/16, N] uint8 (e4m3), global [N] f16; c [M, N] f32 dev, fully
- * overwritten.  N a multiple of 4, K a multiple of 32.  The weight is streamed once per sixteen rows of a.
- * Asynchronous. */
+ * overwritten.  N a multiple of 4, K a multiple of 32 (at most 3136); packed 16-byte aligned, scale 4-byte aligned
+ * (refused otherwise).  More than sixteen rows of a are served up to 64 per pass over the weight where N % 16 == 0,
+ * K % 256 == 0, N >= 256 and a, packed and scale are 16-byte aligned; every other call streams the weight once per
+ * sixteen rows.  Asynchronous. */
 FTM_API int ftm_dense_gemv(ftm_handle* h, const void* a, int a_dtype, const void* packed_kmajor_i32, const void* scale_kmajor_u8,
                            const void* global_f16, int32_t m, int32_t n, int32_t k, float* c, void* stream);
 

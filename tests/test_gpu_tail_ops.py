@@ -288,3 +288,22 @@ def test_dense_gemv_rejects_shapes_it_was_not_built_for():
         moe.dense_gemv(bf16_dev(a), torch.from_numpy(pk.view(np.int32)).to(dev()), torch.from_numpy(sk).to(dev())[:2],
                        torch.from_numpy(glob.view(np.int16)).to(dev()))
     moe.close()
+
+
+def test_dense_gemv_refuses_a_bank_it_cannot_load():
+    """The packed words of four rows are read by one 128-bit load and their scales by one 32-bit load: a bank that starts
+    elsewhere is refused on the host, whatever the number of rows."""
+    m, n, k = 17, 272, 256
+    a, pk, sk, glob = _gemv_case(m, n, k, 6)
+    moe = tiny_handle(64)
+    x, gl = bf16_dev(a), torch.from_numpy(glob.view(np.int16)).to(dev())
+    words, scales = torch.zeros(pk.size + 4, dtype=torch.int32, device=dev()), torch.zeros(sk.size + 4, dtype=torch.uint8, device=dev())
+    good_w, good_s = words[:pk.size].view(k // 8, n), scales[:sk.size].view(k // 16, n)
+    for off in (1, 2, 3):
+        with pytest.raises(pkg.MoEError, match="aligned"):
+            moe.dense_gemv(x, words[off:off + pk.size].view(k // 8, n), good_s, gl)
+        with pytest.raises(pkg.MoEError, match="aligned"):
+            moe.dense_gemv(x, good_w, scales[off:off + sk.size].view(k // 16, n), gl)
+    moe.dense_gemv(x, good_w, good_s, gl)
+    moe.sync_status()
+    moe.close()
