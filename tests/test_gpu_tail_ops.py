@@ -186,9 +186,9 @@ def test_dense_gemv_matches_reference_fixture(case):
                                    (40, 32, 256), (1, 448, 256), (3, 1056, 512), (12, 2000, 2048), (20, 464, 768)])
 def test_dense_gemv_ragged_shapes_against_cpu_path(m, n, k):
     """Rows that are not a multiple of the 32-row tile, K with and without the two-way split, one to several
-    token tiles and more than sixteen tokens (several passes over the weight).  The last four shapes (N a
-    multiple of 16 and at least 448, K a multiple of 256) take the TMA-fed kernel: one tile exactly, a last
-    tile of 160 and of 208 rows, a last tile of 16 rows."""
+    token tiles and more than sixteen tokens (several passes over the weight).  (3, 1056, 512) and (12, 2000, 2048) take the
+    TMA-fed kernel (N a multiple of 16 and at least 672, K a multiple of 256), with last tiles of 384 and 656 rows;
+    (20, 464, 768) the tensor-memory kernel, the others the register-streaming one."""
     a, pk, sk, glob = _gemv_case(m, n, k, 1000 + m + n + k)
     moe = tiny_handle(64)
     got = _run_gemv(moe, a, pk, sk, glob)
@@ -231,16 +231,16 @@ def test_dense_gemv_lm_head_size(m):
                                    (63, 384, 2048), (64, 65552, 256), (65, 272, 512), (81, 512, 256), (130, 304, 768)])
 def test_dense_gemv_many_tokens_against_cpu_path(m, n, k, dtype):
     """More than sixteen tokens with N % 16 == 0, K % 256 == 0: the tensor-memory kernel.  Token counts either side of its
-    16-token and 32-token steps and of the 64 of one pass (a remainder of one goes to the other kernel, 17 and more
-    to a second pass), a last unit of 16 rows, one without its second tile, more units than SMs, two to sixteen chunks
+    16-token and 32-token steps and of the 64 of one pass (a remainder of one goes to the register-streaming kernel at
+    these N, 17 and more to a second pass), a last unit of 16 rows, one without its second tile, more units than SMs, two to sixteen chunks
     of K.  f32 activations keep eleven bits each (half an ulp: 2^-12 relative), independent errors over K products, so
     the row error stays below 2^-12; bf16 activations are exact."""
     a, pk, sk, glob = _gemv_case(m, n, k, 77 + m + n + k)
     x = o.bf16_bits_to_f32(a).copy()
     if dtype == "f32":
         x *= 1.0 + np.random.default_rng(m).uniform(0, 2.0 ** -8, x.shape).astype(np.float32)
-    x[m // 2] *= 2.0 ** -20          # rows of very different size, one of zeros
-    x[m - 1] = 0.0
+    x[m // 2] *= 2.0 ** -20          # rows of very different size, one of zeros (not the last: it may be the remainder)
+    x[1] = 0.0
     moe = tiny_handle(64)
     t = torch.from_numpy(x).to(dev())
     c = moe.dense_gemv(t if dtype == "f32" else t.to(torch.bfloat16), torch.from_numpy(pk.view(np.int32)).to(dev()),
@@ -306,4 +306,49 @@ def test_dense_gemv_refuses_a_bank_it_cannot_load():
             moe.dense_gemv(x, good_w, scales[off:off + sk.size].view(k // 16, n), gl)
     moe.dense_gemv(x, good_w, good_s, gl)
     moe.sync_status()
+    moe.close()
+
+
+def _run_gemv_at(moe, x, pk, sk, glob, a_off=0, s_off=0):
+    """dense_gemv into a buffer of NaNs, with the activations / the scales so many elements into their allocations."""
+    a = torch.zeros(x.numel() + a_off, dtype=x.dtype, device=dev())[a_off:].view(x.shape)
+    a.copy_(x)
+    s = torch.zeros(sk.size + s_off, dtype=torch.uint8, device=dev())[s_off:].view(sk.shape)
+    s.copy_(torch.from_numpy(sk))
+    c = torch.full((x.shape[0], pk.shape[1]), float("nan"), dtype=torch.float32, device=dev())
+    moe.dense_gemv(a, torch.from_numpy(pk.view(np.int32)).to(dev()), s, torch.from_numpy(glob.view(np.int16)).to(dev()), c=c)
+    moe.sync_status()
+    return c.cpu().numpy()
+
+
+@pytest.mark.parametrize("m", [65, 72, 73, 80, 144])
+@pytest.mark.parametrize("n,k", [(688, 512), (1360, 2048)])
+def test_dense_gemv_remainder_after_passes_of_64(m, n, k):
+    """One to sixteen tokens left after passes of 64, N >= 672: the TMA-fed kernel, both token tiles, from token 64 and 128
+    on.  Every element is written (the output starts as NaN) and no token is taken for another (rows differ by powers of two)."""
+    a, pk, sk, glob = _gemv_case(m, n, k, 900 + m + n)
+    x = o.bf16_bits_to_f32(a) * 2.0 ** (np.arange(m, dtype=np.float32)[:, None] % 7)
+    moe = tiny_handle(64)
+    got = _run_gemv_at(moe, torch.from_numpy(x).to(dev()).to(torch.bfloat16), pk, sk, glob)
+    want = o.nvfp4_dense_gemv(x, pk, sk, glob.view(np.uint16))
+    for i in range(m):
+        assert np.linalg.norm(got[i] - want[i]) <= 1e-5 * np.linalg.norm(want[i]), i
+    moe.close()
+
+
+@pytest.mark.parametrize("dtype", ["bf16", "f32"])
+@pytest.mark.parametrize("a_off,s_off", [(1, 0), (4, 0), (0, 4), (3, 12)])
+def test_dense_gemv_many_tokens_at_other_alignments(a_off, s_off, dtype):
+    """More than sixteen tokens whose activations, or scales, do not start on a 16-byte boundary: the tensor-memory kernel
+    cannot read them, the others serve them sixteen tokens at a time.  (Four f32 elements are 16 bytes: the tensor-memory
+    kernel again.)"""
+    m, n, k = 37, 1056, 512
+    a, pk, sk, glob = _gemv_case(m, n, k, 31 + a_off + s_off)
+    x = o.bf16_bits_to_f32(a)
+    moe = tiny_handle(64)
+    t = torch.from_numpy(x).to(dev())
+    got = _run_gemv_at(moe, t if dtype == "f32" else t.to(torch.bfloat16), pk, sk, glob, a_off, s_off)
+    want = o.nvfp4_dense_gemv(x, pk, sk, glob.view(np.uint16))
+    for i in range(m):
+        assert np.linalg.norm(got[i] - want[i]) <= 1e-5 * np.linalg.norm(want[i]), i
     moe.close()
