@@ -898,8 +898,10 @@ __global__ void scale_repack_kernel(const uint8_t* __restrict__ scale /* the slo
 }
 
 // Plan, gate_up and down are chained with programmatic dependent launch: each sets up under the tail of the one before
-// (a block at one token 49 -> 43 us, 37 tokens 84.5 -> 80.7, 173 tokens 118.7 -> 115.9).  From 64 tokens on it used to
-// lose, because the early-resident CTAs kept the shared expert off the SMs; that is done before they come now.
+// (a block at one token 49 -> 43 us, 37 tokens 84.5 -> 80.7, 173 tokens 118.7 -> 115.9; staged, 64 tokens 100.9 -> 93.3).  In
+// a captured step of 48 to 160 tokens under uniform routing the block is 2 to 4 % better off without (128 tokens 139 against
+// 136 us), under skewed routing and launched one by one it is not (128 tokens 97 against 110 and 139 against 146), so every
+// size is chained.  Beside the tcgen05 shared expert gate_up waits for it first (see the caller).
 constexpr int kDefaultVariant = 14;   // register-streaming kernels, fragment-ordered scales, 256-byte L2 fill
 
 template <bool GATE_UP, int K_, int NT, int OCC, int VAR>

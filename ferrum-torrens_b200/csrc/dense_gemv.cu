@@ -7,9 +7,10 @@
 //   scale  [K/16, N] uint8  e4m3 block scale of block b of row n at (b, n)
 //   global [N] f16
 // 248 320 x 2048 is 254 MB of packed bytes and 32 MB of scales, streamed once per step: a pure
-// HBM-bandwidth kernel.  Two kernels share the fragment mapping below: a register-streaming one (any N % 4,
-// K % 32) and, for N % 16 == 0 and K % 256 == 0, one fed by tiled TMA through a shared-memory ring, which is
-// the one the lm_head takes (2.3 times the rate of the first on that shape).
+// HBM-bandwidth kernel.  Three kernels: two share the fragment mapping below and serve sixteen tokens per pass, a
+// register-streaming one (any N % 4, K % 32) and, for N % 16 == 0, K % 256 == 0 and N >= 672, one fed by tiled TMA through a
+// shared-memory ring, which is the one the lm_head takes (2.3 times the rate of the first on that shape); the third, for
+// more tokens, runs on the 5th-generation tensor cores, up to 64 tokens per pass.
 //
 // Work item: 32 consecutive rows (n) x one half of K.  In a K-major bank four consecutive rows of one k-word
 // are 16 contiguous bytes, so lane (g8, t4) of a warp loads, per step, k-word 4*s + t4 of rows
@@ -41,7 +42,7 @@ struct DenseArgs {
     const uint32_t* packed;  // [K/8, N]
     const uint8_t* scale;    // [K/16, N]
     const uint16_t* global;  // [N]
-    float* c;                // [M, N], cleared before the launch
+    float* c;                // [M, N]; cleared before a launch that splits K (not for the tensor-memory kernel)
     int M, N, K, tok0, ntok, splits;
     int32_t* err;
 };
@@ -454,7 +455,10 @@ bool make_plain_map(CUtensorMap* map, CUtensorMapDataType type, int esize, const
 // Consecutive 64-k steps go to different accumulators in turn (two for 64 tokens, four for 32), summed in f32 by the
 // epilogue: the chain of one accumulator stays short, as in the kernels above.
 // Every mbarrier wait is bounded; a wait that gives up raises the error flag and the CTA drains.
-constexpr int kUmmaMinTok = 16;   // sixteen tokens are one pass of either kernel: 97.8 us above, 101.6 us here
+// Seventeen tokens would be two passes of the kernels above; sixteen are one pass of either.  248 320 rows, cold: 99.4 us above
+// and 96.7 here for sixteen tokens, 90.8 and 101.7 for nine.  Smaller banks lean further to this side (75 776 rows 45.8 and
+// 30.9, 8192 rows 26.3 and 16.4 for sixteen), which the border does not use yet.
+constexpr int kUmmaMinTok = 16;
 constexpr int kUmThreads = 768;
 constexpr int kUmTok = 64;                     // most tokens per pass
 constexpr int kUmXStages = 8, kUmRawStages = 6;

@@ -610,8 +610,8 @@ int launch_router_logits(const __nv_bfloat16* x, const __nv_bfloat16* gate_w, in
         c.end();
         return 1;
     }
-    // The wide kernel from 768 tokens (below, its 64 x 32 tiles leave SMs idle: 512 tokens 31.5 us against 49), except
-    // where its tiles just miss one per SM and most SMs would wait for a second round: 1500 tokens (188 tiles) take
+    // The wide kernel from 768 tokens (below, its 64 x 32 tiles leave SMs idle: 512 tokens 31.5 us against 49; from 593
+    // tokens on, two narrow tiles per SM take 51 to 53 us and it would still win by 2 to 4), except where its tiles just miss one per SM and most SMs would wait for a second round: 1500 tokens (188 tiles) take
     // 69.5 us with the narrow kernel, 83 with the wide one; 2048 (256 tiles) 92 against 83.5.
     const dim3 grid((experts + kBE - 1) / kBE, (tokens + kBT - 1) / kBT);
     const int tiles = (int)(grid.x * grid.y);
