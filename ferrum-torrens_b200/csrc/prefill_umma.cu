@@ -297,15 +297,15 @@ umma_grouped_gemm_kernel(const __grid_constant__ XMaps xmaps, const __grid_const
         }
         for (int s = 0; s < kRS; s++) {
             mbar_init(RAW_FULL(s), 1);
-            mbar_init(RAW_EMPTY(s), 8);       // two pieces x four warps
+            mbar_init(RAW_EMPTY(s), 256);
         }
         for (int s = 0; s < kWBufs; s++) {
-            mbar_init(W_READY(s), 4);
+            mbar_init(W_READY(s), 128);
             mbar_init(W_FREE(s), 1);
         }
         for (int s = 0; s < 2; s++) {
             mbar_init(ACC_FULL(s), 2);
-            mbar_init(ACC_EMPTY(s), kEpiSets * 4);
+            mbar_init(ACC_EMPTY(s), kEpiSets * 128);
         }
         *s_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -450,7 +450,7 @@ umma_grouped_gemm_kernel(const __grid_constant__ XMaps xmaps, const __grid_const
                 const int c = w >> 1;
                 const uint32_t stage = stage0 + 2 * (c >> 1) + (w & 1);      // the raw stage holds chunks c & ~1 and c | 1
                 const int st = stage % kRS;
-                ok = mbar_wait_warp(RAW_FULL(st), (stage / kRS) & 1, s_abort, a.err);
+                ok = mbar_wait(RAW_FULL(st), (stage / kRS) & 1, s_abort, a.err);
                 if (!ok) break;
                 const int wb = item % kWBufs;
                 const uint32_t taddr = tlane + wb * kWCols;
@@ -479,7 +479,7 @@ umma_grouped_gemm_kernel(const __grid_constant__ XMaps xmaps, const __grid_const
                 uint32_t r0[16], r1[16];
                 convert(0, r0);
                 convert(1, r1);
-                ok = mbar_wait_warp(W_FREE(wb), ((item / kWBufs) & 1) ^ 1, s_abort, a.err);
+                ok = mbar_wait(W_FREE(wb), ((item / kWBufs) & 1) ^ 1, s_abort, a.err);
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 tmem_st16(taddr, r0);
@@ -488,10 +488,10 @@ umma_grouped_gemm_kernel(const __grid_constant__ XMaps xmaps, const __grid_const
                 tmem_st16(taddr + 32, r0);
                 convert(3, r1);
                 tmem_st16(taddr + 48, r1);
-                mbar_arrive_warp(RAW_EMPTY(st));
+                mbar_arrive(RAW_EMPTY(st));
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                mbar_arrive_warp(W_READY(wb));
+                mbar_arrive(W_READY(wb));
             }
             if (!ok) break;
         }
@@ -523,7 +523,7 @@ umma_grouped_gemm_kernel(const __grid_constant__ XMaps xmaps, const __grid_const
                     }
                     fac[q] = f;
                 }
-                if (!mbar_wait_warp(ACC_FULL(acc.slot), acc.parity(), s_abort, a.err)) break;
+                if (!mbar_wait(ACC_FULL(acc.slot), acc.parity(), s_abort, a.err)) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 {
                     const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + kAccCol0 + r * kTileTok + acc.slot * kAccSlot;
@@ -559,7 +559,7 @@ umma_grouped_gemm_kernel(const __grid_constant__ XMaps xmaps, const __grid_const
                     }
                 }
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                mbar_arrive_warp(ACC_EMPTY(acc.slot));
+                mbar_arrive(ACC_EMPTY(acc.slot));
             }
     
         } else {
@@ -654,7 +654,7 @@ umma_grouped_gemm_kernel(const __grid_constant__ XMaps xmaps, const __grid_const
                     }
                 }
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                mbar_arrive_warp(ACC_EMPTY(acc.slot));
+                mbar_arrive(ACC_EMPTY(acc.slot));
             }
     
         }

@@ -22,8 +22,8 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-// One arrival for a whole converged warp.  The lanes' arrivals on one barrier are served one after the other, and the
-// GEMMs had 256 of them per weight piece (1000 staged tokens 200 -> 191 us, 64 tokens through the lm_head 131 -> 128).
+// One arrival for a whole converged warp (the tensor-memory GEMV: 64 tokens through the lm_head 124.7 -> 123.7 us, 17 tokens
+// 101.8 -> 102.5 against one per lane; in the grouped GEMM it lost, 1000 staged tokens 193.5 -> 195.2, and is not used).
 __device__ __forceinline__ void mbar_arrive_warp(uint32_t bar) {
     __syncwarp();
     if ((threadIdx.x & 31) == 0) mbar_arrive(bar);
