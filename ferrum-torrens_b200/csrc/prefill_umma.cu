@@ -899,10 +899,10 @@ int launch_prefill_umma(const BankView& b, const void* x, int x_dtype, const Dec
     c.begin(K_PERMUTE_ACT);
     // the gather and both GEMMs are launched programmatically behind the kernel before (each waits for it before its first
     // read): 2 to 3 us less between two of them
-    // A token's routes go to one warp from 4096 tokens on and to up to eight below, for warps on every SM.  Staged tokens, 1 / 2
-    // / 4 / 8 warps: 512 99.3 / 97.4 / 97.2 / 98.6 us, 1024 134.6 / 135.2 / 137.0 / 139.2, 2048 211.4 / 214.9 / 215.1 / 219.9: the
-    // steps lie a little high.
-    const int parts = std::min(top_k, tokens >= 4096 ? 1 : tokens >= 2048 ? 2 : tokens >= 1024 ? 4 : 8);
+    // A token's routes go to 1, 2, 4 or 8 warps, about a thousand warps in all: more read and convert the row more often,
+    // fewer leave SMs short of warps.  Staged tokens, captured, 1 / 2 / 4 / 8 warps: 320 92.5 / 91.2 / 90.4 / 91.8 us, 512 99.3 /
+    // 97.4 / 97.2 / 98.6, 1024 134.6 / 135.2 / 137.0 / 139.2, 1300 166.8 / 166.3 / 167.1 / 168.9, 2048 211.4 / 214.9 / 215.1 / 219.9
+    const int parts = std::min(top_k, tokens >= 2048 ? 1 : tokens >= 512 ? 2 : tokens >= 256 ? 4 : 8);
     launch_pdl(prefill_gather_kernel, dim3((unsigned)(((size_t)tokens * parts + 7) / 8)), dim3(256), 0, c.s, x, x_dtype,
                bins_of_route, nbins, (const int32_t*)sc.pos_of_route, tokens, top_k, parts, b.hidden, sc.xg, sc.row_scale);
     c.end();
